@@ -15,25 +15,24 @@
  * Exactness of the int32 sums: |digit| <= 127 and a diagonal holds at most 8 pairs, so a K range
  * of at most 16384 keeps |D_d| < 8 * 16384 * 127^2 < 2^31; longer K runs in chunks of 16384.
  *
- * Device layout: digit planes dA[s][M][Kp] and dB[s][N][Kp] (int8, K contiguous, Kp = K rounded
- * up to 16, zero padded), exponents ea[M], eb[N] (int32).
+ * Device layout: digit panels, the order in which the GEMM reads them. Rows of op(A) in blocks of 128
+ * and columns of op(B) in blocks of 64, k in blocks of 32: panel (row block, k block) holds all slices
+ * one after the other, each as core matrices of 8 rows x 16 bytes (row group g at 256 g, k half h at
+ * 128 h, row r % 8 at 16 (r % 8)); K zero padded; exponents ea[M], eb[N] (int32).
  *
- * GEMM kernel, two forms (GemmForm): one CTA per 128 x BN tile of C, 6 warps. Warp 0 (one lane)
- * streams (pair, k-block) tiles of both operands into a shared-memory ring with TMA (3-D tensor maps
- * over the digit planes, 128-byte swizzle, out-of-range rows and k read as zero); warp 1 owns all 512
- * tensor-memory columns and one lane issues tcgen05.mma (M=128, N=BN, K=32) per 32-byte K step,
- * committing each stage back to the producer and each finished diagonal to the epilogue; warps 2-5
- * (one tensor-memory lane quarter each) read a finished int32 accumulator with tcgen05.ld, scale it
- * and add it in FP64, then hand it back, so the tensor cores work on diagonal d+1 while diagonal d is
- * being recombined.
- *  - partial form (BN = 128, 6 stages; M*N up to 4096^2): two 128-column accumulators and the tile's
- *    FP64 partial sum (two 32-bit columns per C column) share tensor memory; the partial sum stays
- *    there from diagonal to diagonal (tcgen05.st), so C is read once (beta) at the first diagonal and
- *    written once at the last;
- *  - read-modify-write form (BN = 256, 4 stages; larger products): two 256-column accumulators, each
- *    diagonal added into C. A 256-wide tile needs 25 % fewer operand bytes per MAC; above 4096^2 that
- *    outweighs the per-diagonal C traffic (measured; neither a CTA pair sharing B tiles nor shorter
- *    K ranges per launch were faster).
+ * GEMM kernel: persistent, one CTA per SM, 10 warps, tiles of 128 x 64 of C with ALL anti-diagonals (up to
+ * eight at a time: 8 x 64 = 512 tensor-memory columns) accumulated at once. Per k block a stage takes the A
+ * and the B panel with one bulk copy each; as the B slices lie one after the other, one tcgen05.mma
+ * (M = 128, N = 64 w, K = 32) of A slice sa against the w slices from sb on adds the pairs (sa, sb + i) to
+ * diagonals sa + sb + i. So every digit is read once per tile instead of once per pair, and C once:
+ * 42 KB per 28 pairs of a 32-wide k block at 7 slices, 47 bytes per cycle and SM (128 x 256 tiles, one pair at a
+ * time, took 96, more than the L2 delivers, and added every diagonal into C or tensor memory). Warp 0
+ * copies, warp 1 issues the MMAs, warps 2-9 (two per tensor-memory lane quarter) combine the diagonals of a
+ * finished tile in FP64, smallest weight first, and write C. The MMAs of a tile wait for the epilogue of
+ * the one before (tensor memory is full): about 3 % at K = 4096. More than eight diagonals (no trim) run as
+ * several launches that add into C.
+ * Measured on B200 (whole calls, 7 slices, pairs up to the diagonal, 4096^3): 2549 -> 1776 us, 77 TFLOP/s
+ * FP64-equivalent; the tensor pipe is what bounds it (3.85e12 int8 operations in about 1.4 ms, power-capped).
  * Every mbarrier wait is bounded: a stalled pipeline ends the kernel with an error status (per-call
  * abort word and the library's device error word) instead of a hang.
  */
@@ -41,7 +40,6 @@
 #include "tc_ptx.cuh"
 #include "ozaki_digits.cuh"
 #include <cuda_runtime.h>
-#include <cudaTypedefs.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -51,40 +49,35 @@ namespace {
 using namespace xs_tc;
 using namespace xs_oz;
 
-/* Two forms of the GEMM kernel (GemmForm): 128 x 128 C tiles whose FP64 partial sum stays in tensor
-   memory across anti-diagonals (C read and written once; 6 stages), and 128 x 256 tiles that add each
-   diagonal into C (read-modify-write per diagonal; 4 stages, 25 % fewer operand bytes per MAC). The
-   first is faster up to M*N = 4096^2, the second above (measured on B200). */
-constexpr int kBM = 128, kBK = 128;
-template <bool PARTIAL>
-struct GemmForm {
-  static constexpr int BN = PARTIAL ? 128 : 256, STAGES = PARTIAL ? 6 : 4;
-  static constexpr int ATILE = kBM * kBK, BTILE = BN * kBK;
-  static constexpr uint32_t PART_COL = 2 * BN; /* tensor-memory column of the FP64 partial sum (2 per C column) */
-  static constexpr size_t smem_bytes() {
-    return 1024 /* alignment slack */ + (size_t)STAGES * (ATILE + BTILE) + (2 * STAGES + 4) * sizeof(uint64_t) +
-           16 /* tensor-memory address */ + BN * sizeof(int);
-  }
-};
-constexpr long long kPartialMaxMN = 4096ll * 4096ll; /* largest M*N run by the tensor-memory partial form */
+constexpr int kBM = 128, kBN = 64, kBK = 32;
+constexpr int kSliceA = kBM * kBK, kSliceB = kBN * kBK; /* bytes of one slice of a panel */
 constexpr int kMaxSlices = 8;
-constexpr int kMaxPairs = kMaxSlices * kMaxSlices;
-constexpr int kMaxGroups = 2 * kMaxSlices - 1;
-constexpr int kKChunkBlocks = 16384 / kBK; /* k-blocks per launch: keeps every diagonal's int32 sum exact */
-constexpr int kGemmThreads = 192;
+constexpr int kMaxDiag = 512 / kBN;       /* diagonals in tensor memory at a time */
+constexpr int kMaxStages = 6;
+constexpr int kMaxOps = 3 * kMaxSlices;   /* MMAs per k block */
+constexpr int kKChunkBlocks = 16384 / kBK; /* k blocks per launch: keeps every diagonal's int32 sum exact */
+constexpr int kEpiWarps = 8;
+constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
 constexpr int kGroupM = 8; /* row panels per rasterization group */
 constexpr unsigned kErrOzakiTimeout = 4u; /* device error word bit: an Ozaki pipeline wait timed out */
 
 /* ------------------------------------------------------------------------------ slicing */
 
 /* Row maxima of the biased exponent, rows contiguous in memory: element (r, k) at x[r + k*ld].
-   Grid (ceil(R/256), k-chunks); partial maxima meet in emax[] (zeroed by the caller) by atomicMax. */
+   Grid (ceil(R/256), k-chunks), eight loads in flight per thread; partial maxima meet in emax[] (zeroed by
+   the caller) by atomicMax. */
 __global__ void xs_oz_rowexp_rc(const double* __restrict__ x, long long ld, int R, int K, int kchunk, int* __restrict__ emax) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= R) return;
   const int k0 = blockIdx.y * kchunk, k1 = min(K, k0 + kchunk);
   int e = 0;
-  for (int k = k0; k < k1; ++k) e = max(e, biased_exp(x[r + (long long)k * ld]));
+  for (int k = k0; k < k1; k += 8) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = (k + u < k1) ? x[r + (long long)(k + u) * ld] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) e = max(e, biased_exp(v[u]));
+  }
   if (0 != e) atomicMax(emax + r, e);
 }
 
@@ -100,9 +93,9 @@ __global__ void xs_oz_rowexp_kc(const double* __restrict__ x, long long ld, int 
   if (0 == lane) emax[r] = e;
 }
 
-/* Digits of 16 consecutive k of one row into the planes d[s][r][k0 .. k0+15]. */
-__device__ __forceinline__ void slice16(const double (&v)[16], int erow, int ns, signed char* __restrict__ d, long long plane,
-  long long off) {
+/* Digits of 16 consecutive k of one row into the slices of its panel (16 bytes of a core matrix each),
+   `slice` bytes apart. */
+__device__ __forceinline__ void slice16(const double (&v)[16], int erow, int ns, signed char* __restrict__ d, int slice) {
   unsigned long long al[16];
   unsigned sg[16];
 #pragma unroll
@@ -122,35 +115,41 @@ __device__ __forceinline__ void slice16(const double (&v)[16], int erow, int ns,
       for (int b = 0; b < 4; ++b) x |= ((uint32_t)(slice_digit(al[q * 4 + b], sg[q * 4 + b], s) & 0xFF)) << (8 * b);
       w[q] = x;
     }
-    *reinterpret_cast<uint4*>(d + s * plane + off) = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4*>(d + s * slice) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
-/* Slicing with k contiguous (element (r, k) at x[k + r*ld]): one thread per (row, 16 k). */
+/* Bytes from the start of the digit panels to row r, k group kg (of 16) of slice 0; rb rows per block. */
+__device__ __forceinline__ long long panel_offset(int r, int kg, int Kp, int ns, int rb) {
+  const int blk = r / rb, rr = r - blk * rb;
+  return ((long long)blk * (Kp / kBK) + (kg >> 1)) * ns * (rb * kBK) + (rr >> 3) * 256 + (kg & 1) * 128 + (rr & 7) * 16;
+}
+
+/* Slicing with k contiguous (element (r, k) at x[k + r*ld]): one thread per (row, 16 k), eight rows of one
+   k group side by side, so that they write whole core matrices. */
 __global__ void xs_oz_slice_kc(const double* __restrict__ x, long long ld, int R, int K, int Kp, const int* __restrict__ emax,
-  int ns, signed char* __restrict__ d) {
+  int ns, int rb, signed char* __restrict__ d) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int kg = Kp / 16;
-  if (t >= (long long)R * kg) return;
-  const int r = (int)(t / kg), k0 = (int)(t - (long long)r * kg) * 16;
+  const int ng = Kp / 16, r = (int)(t / (8 * ng)) * 8 + (int)(t & 7), kg = (int)((t >> 3) % ng), k0 = kg * 16;
+  if (r >= R) return;
   const double* const row = x + (long long)r * ld;
   double v[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) v[j] = (k0 + j < K) ? row[k0 + j] : 0.0;
-  slice16(v, emax[r], ns, d, (long long)R * Kp, (long long)r * Kp + k0);
+  slice16(v, emax[r], ns, d + panel_offset(r, kg, Kp, ns, rb), rb * kBK);
 }
 
 /* Slicing with rows contiguous (element (r, k) at x[r + k*ld]): threads of a block run over rows
-   (coalesced reads), blockIdx.y over groups of 16 k. */
+   (coalesced reads, whole core matrices written), blockIdx.y over groups of 16 k. */
 __global__ void xs_oz_slice_rc(const double* __restrict__ x, long long ld, int R, int K, int Kp, const int* __restrict__ emax,
-  int ns, signed char* __restrict__ d) {
+  int ns, int rb, signed char* __restrict__ d) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= R) return;
   const int k0 = blockIdx.y * 16;
   double v[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) v[j] = (k0 + j < K) ? x[r + (long long)(k0 + j) * ld] : 0.0;
-  slice16(v, emax[r], ns, d, (long long)R * Kp, (long long)r * Kp + k0);
+  slice16(v, emax[r], ns, d + panel_offset(r, blockIdx.y, Kp, ns, rb), rb * kBK);
 }
 
 /* C = beta * C (K == 0 or alpha == 0). */
@@ -164,17 +163,20 @@ __global__ void xs_oz_scale_c(double* __restrict__ c, long long ldc, int M, int 
 
 /* ------------------------------------------------------------------------------ GEMM */
 
-struct OzGroup {
-  int p0, p1;  /* pairs [p0, p1) of the pair list */
-  int eshift;  /* -2058 - 7d for diagonal d */
-  int pad;
+/* One MMA of a k block: A slice sa against w B slices from sb on, into the columns of diagonal col; acc = 0
+   writes them, 1 adds to them. */
+struct OzOp {
+  unsigned char sa, sb, w, col, acc;
 };
 
 struct OzGemmArgs {
-  int M, N, kb0, kb1; /* k-blocks [kb0, kb1) of 128 */
-  int ngroups;
-  int first; /* 1: this launch applies beta to C */
+  int M, N, kb0, kb1, KB; /* k blocks [kb0, kb1) of KB */
+  int ns, nstages;
+  int ndiag, eshift;      /* diagonals of the launch, -2058 - 7 d of the first */
+  int first;              /* 1: this launch applies beta to C, later ones add to it */
   double alpha, beta;
+  const unsigned char* dA;
+  const unsigned char* dB;
   const int* ea;
   const int* eb;
   double* C;
@@ -182,86 +184,75 @@ struct OzGemmArgs {
   unsigned* abort; /* per-call abort word (zeroed by the host before the first launch) */
   unsigned* dev_err;
   long long wait_limit; /* bound of every pipeline wait, clock cycles */
-  unsigned char sa[kMaxPairs], sb[kMaxPairs];
-  OzGroup g[kMaxGroups];
+  int nops[2];          /* MMAs of the first k block, of the others */
+  OzOp op[2][kMaxOps];
 };
 
-/* alpha * v * 2^E added to c, exactly scaled by 2^E whenever that is a normal number. */
-__device__ __forceinline__ double add_scaled(double c, int v, int E, double alpha) {
-  double t;
-  if (E >= -1022 && E <= 1023) t = (double)v * __longlong_as_double((long long)(E + 1023) << 52);
-  else t = ldexp((double)v, E);
-  return fma(alpha, t, c);
+/* Shared memory: 128 bytes of alignment slack, the ring, its barriers, the tensor-memory address. */
+__host__ __device__ constexpr size_t oz_gemm_smem(int ns, int stages) {
+  return 128 + (size_t)stages * ns * (kSliceA + kSliceB) + (2 * kMaxStages + 2) * sizeof(uint64_t) + 16;
 }
 
-template <bool PARTIAL>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-  xs_ozaki_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-    const __grid_constant__ OzGemmArgs args) {
-  using F = GemmForm<PARTIAL>;
-  constexpr int kBN = F::BN, kStages = F::STAGES, kATileBytes = F::ATILE, kBTileBytes = F::BTILE;
-  constexpr uint32_t kPartCol = F::PART_COL;
-  extern __shared__ unsigned char smem_raw[];
-  unsigned char* const smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  unsigned char* const sA = smem;
-  unsigned char* const sB = smem + kStages * kATileBytes;
-  uint64_t* const bars = (uint64_t*)(sB + kStages * kBTileBytes);
-  uint64_t* const full = bars;
-  uint64_t* const empty = bars + kStages;
-  uint64_t* const accf = bars + 2 * kStages;
-  uint64_t* const acce = accf + 2;
-  uint32_t* const tmem_slot = (uint32_t*)(acce + 2);
-  int* const s_eb = (int*)(tmem_slot + 4);
-  unsigned* const abort = args.abort;
+/* Tile t: groups of kGroupM row panels sweep the column panels together, so that the CTAs running at one
+   time share their panels in L2. */
+__device__ __forceinline__ void oz_tile(int t, int ntm, int ntn, int& bm, int& bn) {
+  const int per_group = kGroupM * ntn, g = t / per_group, first = g * kGroupM;
+  const int gsize = min(kGroupM, ntm - first), r = t - g * per_group;
+  bm = first + r % gsize;
+  bn = r / gsize;
+}
 
+__global__ void __launch_bounds__(kGemmThreads, 1) xs_ozaki_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* const smem = (unsigned char*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
+  const int ns = args.ns, nst = args.nstages;
+  const uint32_t abytes = (uint32_t)(ns * kSliceA), bbytes = (uint32_t)(ns * kSliceB), stage_bytes = abytes + bbytes;
+  uint64_t* const bars = (uint64_t*)(smem + (size_t)nst * stage_bytes);
+  uint64_t* const full = bars;
+  uint64_t* const empty = bars + kMaxStages;
+  uint64_t* const accf = bars + 2 * kMaxStages;
+  uint64_t* const acce = accf + 1;
+  uint32_t* const tmem_slot = (uint32_t*)(acce + 1);
+  unsigned* const abort = args.abort;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  /* tile order: groups of kGroupM row panels sweep the column panels together, so that the CTAs of
-     one wave share their A row panels and B column panels in L2 */
-  int n0, m0;
-  {
-    const int ntm = (args.M + kBM - 1) / kBM, ntn = (args.N + kBN - 1) / kBN;
-    const int id = blockIdx.x, per_group = kGroupM * ntn, g = id / per_group, first = g * kGroupM;
-    const int gsize = min(kGroupM, ntm - first), r = id - g * per_group;
-    m0 = (first + r % gsize) * kBM;
-    n0 = (r / gsize) * kBN;
-  }
+  const int ntm = (args.M + kBM - 1) / kBM, ntn = (args.N + kBN - 1) / kBN, ntiles = ntm * ntn;
   if (0 == threadIdx.x) {
-    for (int i = 0; i < kStages; ++i) {
+    for (int i = 0; i < nst; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&accf[i], 1);
-      mbar_init(&acce[i], 128);
-    }
+    mbar_init(accf, 1);
+    mbar_init(acce, 32 * kEpiWarps);
     fence_barrier_init();
-    prefetch_tensormap(&mapA);
-    prefetch_tensormap(&mapB);
   }
   if (1 == warp) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  for (int j = threadIdx.x; j < kBN; j += blockDim.x) s_eb[j] = (n0 + j < args.N) ? args.eb[n0 + j] : 0;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (0 == warp) { /* TMA producer */
+  if (0 == warp) { /* producer */
     if (0 == lane) {
-      int it = 0;
+      int stage = 0;
+      uint32_t ph = 0u;
       bool ok = true;
-      for (int g = 0; g < args.ngroups && ok; ++g) {
-        for (int p = args.g[g].p0; p < args.g[g].p1 && ok; ++p) {
-          const int za = args.sa[p], zb = args.sb[p];
-          for (int kb = args.kb0; kb < args.kb1; ++kb, ++it) {
-            const int stage = it % kStages;
-            const uint32_t ph = (uint32_t)(it / kStages) & 1u;
-            if (!(ok = mbar_wait(&empty[stage], ph ^ 1u, abort, 1u, args.wait_limit))) break;
-            mbar_arrive_expect_tx(&full[stage], kATileBytes + kBTileBytes);
-            tma_load_3d(sA + stage * kATileBytes, &mapA, kb * kBK, m0, za, &full[stage]);
-            tma_load_3d(sB + stage * kBTileBytes, &mapB, kb * kBK, n0, zb, &full[stage]);
+      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+        int bm, bn;
+        oz_tile(t, ntm, ntn, bm, bn);
+        const unsigned char* const pa = args.dA + (size_t)bm * args.KB * abytes;
+        const unsigned char* const pb = args.dB + (size_t)bn * args.KB * bbytes;
+        for (int kb = args.kb0; kb < args.kb1; ++kb) {
+          if (!(ok = mbar_wait(&empty[stage], ph ^ 1u, abort, 1u, args.wait_limit))) break;
+          unsigned char* const st = smem + (size_t)stage * stage_bytes;
+          mbar_arrive_expect_tx(&full[stage], stage_bytes);
+          bulk_load(st, pa + (size_t)kb * abytes, abytes, &full[stage]);
+          bulk_load(st + abytes, pb + (size_t)kb * bbytes, bbytes, &full[stage]);
+          if (++stage == nst) {
+            stage = 0;
+            ph ^= 1u;
           }
         }
       }
@@ -269,134 +260,78 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   }
   else if (1 == warp) { /* MMA issuer */
     if (0 == lane) {
-      const uint32_t idesc = idesc_i8(kBM, kBN);
-      int it = 0;
+      int stage = 0;
+      uint32_t ph = 0u, use = 0u;
       bool ok = true;
-      for (int g = 0; g < args.ngroups && ok; ++g) {
-        const int buf = g & 1, use = g >> 1;
-        if (!(ok = mbar_wait(&acce[buf], ((uint32_t)use & 1u) ^ 1u, abort, 2u, args.wait_limit))) break;
+      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++use) {
+        if (!(ok = mbar_wait(acce, (use & 1u) ^ 1u, abort, 2u, args.wait_limit))) break;
         tc_fence_after();
-        const uint32_t d = tmem + (uint32_t)(buf * kBN);
-        uint32_t acc = 0;
-        for (int p = args.g[g].p0; p < args.g[g].p1 && ok; ++p) {
-          for (int kb = args.kb0; kb < args.kb1; ++kb, ++it) {
-            const int stage = it % kStages;
-            const uint32_t ph = (uint32_t)(it / kStages) & 1u;
-            if (!(ok = mbar_wait(&full[stage], ph, abort, 2u, args.wait_limit))) break;
-            tc_fence_after();
-            const uint32_t a0 = smem_u32(sA + stage * kATileBytes), b0 = smem_u32(sB + stage * kBTileBytes);
-#pragma unroll
-            for (int kk = 0; kk < kBK / 32; ++kk) {
-              mma_i8(d, desc_k_sw128(a0 + kk * 32), desc_k_sw128(b0 + kk * 32), idesc, acc);
-              acc = 1;
-            }
-            mma_commit(&empty[stage]);
+        for (int kb = args.kb0; kb < args.kb1; ++kb) {
+          if (!(ok = mbar_wait(&full[stage], ph, abort, 2u, args.wait_limit))) break;
+          tc_fence_after();
+          const uint32_t a0 = smem_u32(smem + (size_t)stage * stage_bytes), b0 = a0 + abytes;
+          const int which = (kb == args.kb0) ? 0 : 1, n = args.nops[which];
+          for (int i = 0; i < n; ++i) {
+            const OzOp& o = args.op[which][i];
+            mma_i8(tmem + (uint32_t)(o.col * kBN), desc_k_noswz(a0 + o.sa * kSliceA, 128, 256),
+              desc_k_noswz(b0 + o.sb * kSliceB, 128, 256), idesc_i8(kBM, o.w * kBN), o.acc);
+          }
+          mma_commit(&empty[stage]);
+          if (++stage == nst) {
+            stage = 0;
+            ph ^= 1u;
           }
         }
-        if (ok) mma_commit(&accf[buf]);
+        if (ok) mma_commit(accf);
       }
     }
   }
-  else if constexpr (PARTIAL) { /* epilogue: warps 2..5, tensor-memory lane quarter warp % 4; this lane's row
-                                   of the tile keeps its FP64 partial sum in tensor memory across diagonals */
-    const int q = warp & 3;
-    const int row = m0 + q * 32 + lane;
-    const bool rok = row < args.M;
-    const int ear = rok ? args.ea[row] : 0;
-    const uint32_t tlane = tmem + ((uint32_t)(q * 32) << 16);
-    const bool read_c = (0 == args.first) || 0.0 != args.beta;
-    for (int g = 0; g < args.ngroups; ++g) {
-      const int buf = g & 1, use = g >> 1;
-      if (!mbar_wait(&accf[buf], (uint32_t)use & 1u, abort, 8u, args.wait_limit)) break;
+  else { /* epilogue: tensor-memory lane quarter warp % 4, column half (warp - 2) / 4; thread = one row, 32 columns */
+    const int q = warp & 3, cb = ((warp - 2) >> 2) * 32;
+    const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cb;
+    uint32_t use = 0u;
+    const double w_last = __longlong_as_double((long long)(1023 - 7 * (args.ndiag - 1)) << 52);
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++use) {
+      int bm, bn;
+      oz_tile(t, ntm, ntn, bm, bn);
+      const int row = bm * kBM + q * 32 + lane, n0 = bn * kBN + cb;
+      const bool rok = row < args.M;
+      const int er = (rok ? args.ea[row] : 0) + args.eshift, ec = (n0 + lane < args.N) ? args.eb[n0 + lane] : 0;
+      if (!mbar_wait(accf, use & 1u, abort, 8u, args.wait_limit)) break;
       tc_fence_after();
-      const int eshift = args.g[g].eshift;
-      const bool first_g = (0 == g), last_g = (g + 1 == args.ngroups);
-      for (int c0 = 0; c0 < kBN; c0 += 16) {
-        uint32_t v[16], pw[32];
-        tmem_ld16(tlane + (uint32_t)(buf * kBN + c0), v);
-        if (!first_g) tmem_ld32(tlane + kPartCol + (uint32_t)(2 * c0), pw);
-        tmem_ld_wait();
-        const int ncol = min(16, args.N - (n0 + c0));
-        double* const crow = args.C + row + (long long)(n0 + c0) * args.ldc;
-        double part[16];
-        if (first_g) { /* the partial sum starts as beta * C (the call's first launch) or C (a later K range) */
+      double sum[32];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) part[j] = (rok && j < ncol && read_c) ? crow[(long long)j * args.ldc] : 0.0;
-          if (0 != args.first) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) part[j] *= args.beta;
-          }
-        }
-        else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) part[j] = __hiloint2double((int)pw[2 * j + 1], (int)pw[2 * j]);
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int iv = (int)v[j];
-          if (0 != iv) part[j] = add_scaled(part[j], iv, ear + s_eb[c0 + j] + eshift, args.alpha);
-        }
-        if (last_g) {
-          if (rok) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              if (j < ncol) crow[(long long)j * args.ldc] = part[j];
-            }
-          }
-        }
-        else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            pw[2 * j] = (uint32_t)__double2loint(part[j]);
-            pw[2 * j + 1] = (uint32_t)__double2hiint(part[j]);
-          }
-          tmem_st32(tlane + kPartCol + (uint32_t)(2 * c0), pw);
-        }
-      }
-      if (!last_g) tmem_st_wait(); /* the partial sums are in tensor memory before the next diagonal reads them */
-      tc_fence_before();
-      mbar_arrive(&acce[buf]);
-    }
-  }
-  else { /* epilogue: warps 2..5, tensor-memory lane quarter warp % 4; each diagonal is added into C */
-    const int q = warp & 3;
-    const int row = m0 + q * 32 + lane;
-    const bool rok = row < args.M;
-    const int ear = rok ? args.ea[row] : 0;
-    const uint32_t tlane = tmem + ((uint32_t)(q * 32) << 16);
-    for (int g = 0; g < args.ngroups; ++g) {
-      const int buf = g & 1, use = g >> 1;
-      if (!mbar_wait(&accf[buf], (uint32_t)use & 1u, abort, 8u, args.wait_limit)) break;
-      tc_fence_after();
-      const int eshift = args.g[g].eshift;
-      const bool beta_now = (0 != args.first) && (0 == g);
-      for (int c0 = 0; c0 < kBN; c0 += 32) {
+      for (int j = 0; j < 32; ++j) sum[j] = 0.0;
+      double w = w_last;
+      for (int d = args.ndiag - 1; d >= 0; --d, w *= 128.0) {
         uint32_t v[32];
-        tmem_ld32(tlane + (uint32_t)(buf * kBN + c0), v);
+        tmem_ld32(tbase + (uint32_t)(d * kBN), v);
         tmem_ld_wait();
-        if (rok) { /* all 32 loads of the chunk first, then the updates and the stores (no load waits for a
-                      store it cannot be proven independent of) */
-          double* const crow = args.C + row + (long long)(n0 + c0) * args.ldc;
-          const int ncol = min(32, args.N - (n0 + c0));
-          const bool read_c = !beta_now || 0.0 != args.beta;
-          double cv[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) cv[j] = (j < ncol && read_c) ? crow[(long long)j * args.ldc] : 0.0;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            double c = beta_now ? args.beta * cv[j] : cv[j];
-            const int iv = (int)v[j];
-            if (0 != iv) c = add_scaled(c, iv, ear + s_eb[c0 + j] + eshift, args.alpha);
-            cv[j] = c;
-          }
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (j < ncol) crow[(long long)j * args.ldc] = cv[j];
-          }
+        for (int j = 0; j < 32; ++j) { /* exact int32 -> double: 2^52 + 2^31 + v, minus the offset */
+          const double dv = __hiloint2double(0x43300000, (int)(v[j] ^ 0x80000000u)) - 4503601774854144.0;
+          sum[j] = fma(dv, w, sum[j]);
         }
       }
       tc_fence_before();
-      mbar_arrive(&acce[buf]);
+      mbar_arrive(acce); /* the accumulators are read: the next tile's MMAs may start */
+      double* const crow = args.C + row + (long long)n0 * args.ldc;
+      const bool read_c = (0 == args.first) || 0.0 != args.beta;
+      const double beta = (0 != args.first) ? args.beta : 1.0;
+#pragma unroll
+      for (int j0 = 0; j0 < 32; j0 += 8) {
+        double old[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          old[j] = (rok && read_c && n0 + j0 + j < args.N) ? crow[(long long)(j0 + j) * args.ldc] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int E = er + __shfl_sync(0xffffffffu, ec, j0 + j);
+          const double x = sum[j0 + j];
+          const double sc = (E >= -1022 && E <= 1023) ? x * __longlong_as_double((long long)(E + 1023) << 52) : ldexp(x, E);
+          if (rok && n0 + j0 + j < args.N) crow[(long long)(j0 + j) * args.ldc] = fma(args.alpha, sc, read_c ? beta * old[j] : 0.0);
+        }
+      }
     }
   }
   if (0 != *(volatile unsigned*)abort) { /* let copies and MMAs still in flight land before TMEM goes */
@@ -413,50 +348,49 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
 /* ------------------------------------------------------------------------------ host */
 
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn(void) {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (nullptr == fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaSuccess == cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) &&
-        cudaDriverEntryPointSuccess == q) {
-      fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-    }
-  }
-  return fn;
-}
-
-/* 3-D map over digit planes d[s][R][Kp] (int8), box 128 (k) x rows x 1, 128-byte swizzle. */
-int make_plane_map(CUtensorMap* map, const void* base, int Kp, int R, int ns, int box_rows) {
-  const PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
-  if (nullptr == fn) return (int)cudaErrorNotSupported;
-  const cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)R, (cuuint64_t)ns};
-  const cuuint64_t strides[2] = {(cuuint64_t)Kp, (cuuint64_t)Kp * (cuuint64_t)R};
-  const cuuint32_t box[3] = {(cuuint32_t)kBK, (cuuint32_t)box_rows, 1};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
-    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return (CUDA_SUCCESS == r) ? 0 : (int)cudaErrorInvalidValue;
-}
-
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-/* Exponents and digit planes of op(X) viewed as R rows of K entries: element (r, k) at
-   x[r + k*ld] when rows_contiguous, else at x[k + r*ld]. */
-int slice_operand(const double* x, long long ld, bool rows_contiguous, int R, int K, int Kp, int ns, int* emax,
-  signed char* planes, cudaStream_t s) {
+/* Exponents and digit panels of op(X) viewed as R rows of K entries, rb rows per block: element (r, k)
+   at x[r + k*ld] when rows_contiguous, else at x[k + r*ld]. */
+int slice_operand(const double* x, long long ld, bool rows_contiguous, int R, int K, int Kp, int ns, int rb, int* emax,
+  signed char* panels, cudaStream_t s) {
   if (rows_contiguous) {
-    const int kchunk = 256;
-    xs_oz_rowexp_rc<<<dim3((R + 255) / 256, (K + kchunk - 1) / kchunk), 256, 0, s>>>(x, ld, R, K, kchunk, emax);
-    xs_oz_slice_rc<<<dim3((R + 127) / 128, Kp / 16), 128, 0, s>>>(x, ld, R, K, Kp, emax, ns, planes);
+    /* k ranges short enough that small operands fill the device too */
+    const int nrb = (R + 255) / 256, want = 4 * xs_sm_count() / nrb + 1, kchunk = max(16, min(256, (K + want - 1) / want));
+    xs_oz_rowexp_rc<<<dim3(nrb, (K + kchunk - 1) / kchunk), 256, 0, s>>>(x, ld, R, K, kchunk, emax);
+    xs_oz_slice_rc<<<dim3((R + 127) / 128, Kp / 16), 128, 0, s>>>(x, ld, R, K, Kp, emax, ns, rb, panels);
   }
   else {
     xs_oz_rowexp_kc<<<(R + 7) / 8, 256, 0, s>>>(x, ld, R, K, emax);
-    const long long n = (long long)R * (Kp / 16);
-    xs_oz_slice_kc<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(x, ld, R, K, Kp, emax, ns, planes);
+    const long long n = (long long)((R + 7) / 8 * 8) * (Kp / 16);
+    xs_oz_slice_kc<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(x, ld, R, K, Kp, emax, ns, rb, panels);
   }
   return (int)cudaGetLastError();
+}
+
+/* The MMAs of a k block for the diagonals [d0, d0 + nd): per A slice its run of B slices, in pieces of at
+   most four slices (256 columns) of nearly equal width. first: a diagonal's first MMA writes its columns
+   (a piece never mixes written and added columns). */
+int make_ops(int ns, int d0, int nd, bool first, OzOp* op) {
+  int n = 0, fresh = d0; /* diagonals from here on have not been written */
+  for (int sa = 0; sa < ns; ++sa) {
+    const int lo = max(0, d0 - sa), hi = min(ns - 1, d0 + nd - 1 - sa); /* B slices */
+    for (int b = lo; b <= hi;) {
+      const bool acc = !first || sa + b < fresh;
+      int e = hi; /* last slice of the run with the same accumulate flag */
+      if (first && acc && sa + e >= fresh) e = fresh - 1 - sa;
+      const int len = e - b + 1, parts = (len + 3) / 4, w = (len + parts - 1) / parts;
+      op[n].sa = (unsigned char)sa;
+      op[n].sb = (unsigned char)b;
+      op[n].w = (unsigned char)w;
+      op[n].col = (unsigned char)(sa + b - d0);
+      op[n].acc = acc ? 1 : 0;
+      ++n;
+      b += w;
+    }
+    if (lo <= hi) fresh = max(fresh, sa + hi + 1);
+  }
+  return n;
 }
 
 }  // namespace
@@ -464,9 +398,9 @@ int slice_operand(const double* x, long long ld, bool rows_contiguous, int R, in
 extern "C" {
 
 size_t xs_ozaki_gemm_scratch_bytes(int M, int N, int K, int nslices) {
-  const size_t Kp = align_up((size_t)(K > 0 ? K : 1), 16);
-  return align_up((size_t)nslices * M * Kp, 1024) + align_up((size_t)nslices * N * Kp, 1024) + align_up(sizeof(int) * M, 256) +
-         align_up(sizeof(int) * N, 256) + 256;
+  const size_t Kp = align_up((size_t)(K > 0 ? K : 1), kBK);
+  return align_up((size_t)nslices * align_up(M, kBM) * Kp, 1024) + align_up((size_t)nslices * align_up(N, kBN) * Kp, 1024) +
+         align_up(sizeof(int) * M, 256) + align_up(sizeof(int) * N, 256) + 256;
 }
 
 int xs_ozaki_gemm(char transa, char transb, int M, int N, int K, double alpha, const double* a, int lda, const double* b,
@@ -486,12 +420,12 @@ int xs_ozaki_gemm(char transa, char transb, int M, int N, int K, double alpha, c
   if (nullptr == scratch || scratch_bytes < xs_ozaki_gemm_scratch_bytes(M, N, K, nslices)) return (int)cudaErrorInvalidValue;
   const int maxcut = 2 * (nslices - 1);
   if (cutoff < 0 || cutoff > maxcut) cutoff = maxcut;
-  const int Kp = (int)align_up((size_t)K, 16);
+  const int Kp = (int)align_up((size_t)K, kBK);
   char* p = (char*)scratch;
   signed char* const dA = (signed char*)p;
-  p += align_up((size_t)nslices * M * Kp, 1024);
+  p += align_up((size_t)nslices * align_up(M, kBM) * Kp, 1024);
   signed char* const dB = (signed char*)p;
-  p += align_up((size_t)nslices * N * Kp, 1024);
+  p += align_up((size_t)nslices * align_up(N, kBN) * Kp, 1024);
   int* const ea = (int*)p;
   p += align_up(sizeof(int) * M, 256);
   int* const eb = (int*)p;
@@ -502,13 +436,9 @@ int xs_ozaki_gemm(char transa, char transb, int M, int N, int K, double alpha, c
   /* rows of op(A): A(i, k) at a[i + k*lda] ('N') or a[k + i*lda] ('T'); columns of op(B): B(k, j)
      at b[k + j*ldb] ('N', k contiguous) or b[j + k*ldb] ('T') */
   void* prof = xs_profile_begin(stream);
-  if (0 != (r = slice_operand(a, lda, !ta, M, K, Kp, nslices, ea, dA, s))) return r;
-  if (0 != (r = slice_operand(b, ldb, tb, N, K, Kp, nslices, eb, dB, s))) return r;
+  if (0 != (r = slice_operand(a, lda, !ta, M, K, Kp, nslices, kBM, ea, dA, s))) return r;
+  if (0 != (r = slice_operand(b, ldb, tb, N, K, Kp, nslices, kBN, eb, dB, s))) return r;
   xs_profile_end(prof, "ozaki_slice", 0.0, 8.0 * ((double)M * K + (double)K * N), stream);
-  CUtensorMap mapA, mapB;
-  if (0 != (r = make_plane_map(&mapA, dA, Kp, M, nslices, kBM))) return r;
-  const bool partial = (long long)M * N <= kPartialMaxMN;
-  if (0 != (r = make_plane_map(&mapB, dB, Kp, N, nslices, partial ? GemmForm<true>::BN : GemmForm<false>::BN))) return r;
   OzGemmArgs args;
   memset(&args, 0, sizeof(args));
   args.M = M;
@@ -523,39 +453,31 @@ int xs_ozaki_gemm(char transa, char transb, int M, int N, int K, double alpha, c
   args.dev_err = xs_device_error_ptr();
   args.wait_limit = xs_wait_limit();
   if (nullptr == args.dev_err) return (int)cudaErrorInvalidValue;
-  int np = 0, ng = 0;
-  for (int d = 0; d <= cutoff; ++d) { /* pairs ordered by anti-diagonal, one accumulation group each */
-    const int p0 = np;
-    for (int sa = 0; sa < nslices; ++sa) {
-      const int sb = d - sa;
-      if (sb < 0 || sb >= nslices) continue;
-      args.sa[np] = (unsigned char)sa;
-      args.sb[np] = (unsigned char)sb;
-      ++np;
-    }
-    if (np > p0) {
-      args.g[ng].p0 = p0;
-      args.g[ng].p1 = np;
-      args.g[ng].eshift = -2058 - 7 * d;
-      ++ng;
-    }
-  }
-  args.ngroups = ng;
-  const size_t smem = partial ? GemmForm<true>::smem_bytes() : GemmForm<false>::smem_bytes();
-  void (*const kernel)(const CUtensorMap, const CUtensorMap, const OzGemmArgs) =
-    partial ? xs_ozaki_gemm_kernel<true> : xs_ozaki_gemm_kernel<false>;
-  if (0 != (r = xs_func_smem((const void*)kernel, smem))) return r;
-  const int nkb = (K + kBK - 1) / kBK, bn = partial ? GemmForm<true>::BN : GemmForm<false>::BN;
-  const dim3 grid(((N + bn - 1) / bn) * ((M + kBM - 1) / kBM));
-  for (int kb0 = 0; kb0 < nkb; kb0 += kKChunkBlocks) {
+  args.dA = (const unsigned char*)dA;
+  args.dB = (const unsigned char*)dB;
+  args.ns = nslices;
+  args.KB = Kp / kBK;
+  args.nstages = kMaxStages;
+  while (oz_gemm_smem(nslices, args.nstages) > 227 * 1024) --args.nstages;
+  /* at least 120 KB, so that an SM takes one CTA: it owns all tensor-memory columns */
+  const size_t smem = max((size_t)120 * 1024, oz_gemm_smem(nslices, args.nstages));
+  if (0 != (r = xs_func_smem((const void*)xs_ozaki_gemm_kernel, smem))) return r;
+  const int ntiles = ((N + kBN - 1) / kBN) * ((M + kBM - 1) / kBM);
+  for (int kb0 = 0; kb0 < args.KB; kb0 += kKChunkBlocks) {
     args.kb0 = kb0;
-    args.kb1 = (kb0 + kKChunkBlocks < nkb) ? kb0 + kKChunkBlocks : nkb;
-    args.first = (0 == kb0) ? 1 : 0;
-    prof = xs_profile_begin(stream);
-    kernel<<<grid, kGemmThreads, smem, s>>>(mapA, mapB, args);
-    if (0 != (r = (int)cudaGetLastError())) return r;
-    const double kc = (double)(args.kb1 - args.kb0) * kBK;
-    xs_profile_end(prof, "ozaki_gemm", 2.0 * M * N * (kc < K ? kc : K), 0.0, stream);
+    args.kb1 = (kb0 + kKChunkBlocks < args.KB) ? kb0 + kKChunkBlocks : args.KB;
+    for (int d0 = 0; d0 <= cutoff; d0 += kMaxDiag) {
+      args.ndiag = min(kMaxDiag, cutoff + 1 - d0);
+      args.eshift = -2058 - 7 * d0;
+      args.first = (0 == kb0 && 0 == d0) ? 1 : 0;
+      args.nops[0] = make_ops(nslices, d0, args.ndiag, true, args.op[0]);
+      args.nops[1] = make_ops(nslices, d0, args.ndiag, false, args.op[1]);
+      prof = xs_profile_begin(stream);
+      xs_ozaki_gemm_kernel<<<min(ntiles, xs_sm_count()), kGemmThreads, smem, s>>>(args);
+      if (0 != (r = (int)cudaGetLastError())) return r;
+      const double kc = (double)(args.kb1 - args.kb0) * kBK;
+      xs_profile_end(prof, "ozaki_gemm", 2.0 * M * N * (kc < K ? kc : K), 0.0, stream);
+    }
   }
   return 0;
 }
