@@ -73,6 +73,7 @@ typedef struct xs_smm_params_t {
   int generic; /* 1: always use the runtime-shape kernel even if a specialised one exists */
   int wpb;     /* warps per CTA */
   int sorted;  /* 1: the stack is known to be grouped by c (skip the device sort) */
+  int tile;    /* 1: not a tuned record, so the tile kernel may take the stack where it is the faster one */
 } xs_smm_params_t;
 
 /** kp value that selects the register-blocked FMA stack kernel (small blocks). */

@@ -24,6 +24,8 @@
  *   The result is bitwise reproducible from run to run, unlike FP atomics.
  */
 #include "internal.h"
+#include "smm_stack.cuh"
+#include "smm_tile.h"
 #include "tc_ptx.cuh"
 #include "../../include/libxstream_b200.h"
 #include <cuda_runtime.h>
@@ -32,88 +34,14 @@
 #include <string.h>
 
 namespace {
+using namespace xs_stack;
 
 /* Warps of the combine kernel (its warp partials go through dynamic shared memory). */
 constexpr int kCombineWarps = 16;
 
-/* Programmatic dependent launch: a kernel launched with pdl_launch may be scheduled while the
-   kernel before it in the stream is still running (once that kernel's CTAs have all passed
-   pdl_trigger or exited); it must call pdl_wait before it reads anything its predecessor writes.
-   Both are no-ops for a kernel launched the ordinary way. */
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" :::); }
-
-template <typename... KArgs, typename... Args>
-cudaError_t pdl_launch(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
-/* Release/acquire fence at GPU scope: orders this thread's piece stores before its (relaxed) arrival
-   increment, and a CTA's reads of the other CTAs' pieces after the increment that found them all
-   published. Lighter than the sequentially consistent __threadfence(). */
-__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-
-/* Bring a block of `count` contiguous doubles into L2 (one prefetch per 128-byte line, by 32 lanes). */
-__device__ __forceinline__ void prefetch_block_l2(const double* p, int count, int lane) {
-  for (int x = 16 * lane; x < count + 15; x += 16 * 32) {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (x < count ? x : count - 1)));
-  }
-}
-
-__device__ __forceinline__ void dmma_m8n8k4(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
-
-/* Per-lane geometry of a warp sub-tile (8*MT x 8*NT of C): which fragment rows/columns it loads. */
-template <int MT, int NT>
-struct Tile {
-  bool rok[MT], cok[NT];
-  int r0, c0;
-  __device__ __forceinline__ void init(int sub, int nsub_n, int m, int n, int g) {
-    const int sm = sub / nsub_n, sn = sub - sm * nsub_n;
-    r0 = sm * 8 * MT;
-    c0 = sn * 8 * NT;
-#pragma unroll
-    for (int i = 0; i < MT; ++i) rok[i] = r0 + 8 * i + g < m;
-#pragma unroll
-    for (int j = 0; j < NT; ++j) cok[j] = c0 + 8 * j + g < n;
-  }
-};
-
-/* Write-back of a finished C sub-tile: each element has exactly one writer (red.global.add.f64). */
-template <int MT, int NT>
-__device__ __forceinline__ void commit_tile(double* __restrict__ C, size_t coff, const double (&acc)[MT][NT][2], int m,
-  int n, int g, int t, const Tile<MT, NT>& tl, double alpha) {
-#pragma unroll
-  for (int i = 0; i < MT; ++i) {
-    const int r = tl.r0 + 8 * i + g;
-    if (r < m) {
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const int cc = tl.c0 + 8 * j + 2 * t;
-        if (cc < n) atomicAdd(C + coff + (size_t)cc * m + r, alpha * acc[i][j][0]);
-        if (cc + 1 < n) atomicAdd(C + coff + (size_t)(cc + 1) * m + r, alpha * acc[i][j][1]);
-      }
-    }
-  }
-}
-
 /* How a warp holds its C sub-tile, for the merge and combine code that sums pieces ([REGS][32]
    doubles, element r of lane l at r * 32 + l) and writes a finished sum back: the DMMA fragments of an
    8*MT x 8*NT sub-tile (element (i, j, h) at (i * NT + j) * 2 + h). */
-struct StackTask;
 template <int MT, int NT>
 struct DmmaLayout {
   static constexpr int REGS = MT * NT * 2;
@@ -136,33 +64,6 @@ __host__ __device__ constexpr int smm_min_blocks(int mt, int nt) { return (mt * 
    a segment that ends inside the chunk is written back at once; pieces of segments crossing chunk
    boundaries are merged inside the CTA through shared memory in warp order, and only segments that
    cross the CTA's own boundaries leave a CTA-level piece in global scratch for the combine kernel. */
-/* What the stack kernel needs to know about one stack: one task for a single call, one per stack
-   for a batch. keys/vals are the stack's grouped entries, pieces its CTA-level piece slots. */
-struct StackTask {
-  const double* a;
-  const double* b;
-  double* c;
-  const unsigned* keys;
-  const unsigned long long* vals;
-  double* pieces;
-  int S, m, n, k;
-  int L, nchunks, ngroups, nsub_n, nsub;
-  int item_begin; /* first work item of this stack (batch) */
-  int cls;        /* tile class (MT - 1) * 4 + (NT - 1) (batch) */
-  int sid;        /* stack index within the call: tag of its segment-list entries */
-  int kind;       /* unified batch kernel: 0 = register kernel of tile class cls, else 1 + staged shape index */
-  double alpha;   /* C += alpha * A * B (1 for the LIBSMM ABI) */
-  int* arrive;    /* per (CTA group, sub-tile) arrival counters of CTA-crossing segments, zero at launch:
-                     the stack kernel combines them itself; nullptr: they go to the combine kernel */
-  const int* raw; /* the caller's parameter stack (input of the grouping), for the L2 prefetch */
-  int rstride;    /* ints per parameter record (3 or 6) */
-  int rbase;      /* a-offset position within a record (b follows) */
-  int rshift;     /* added to a record's offsets to make them 0-based (-1: 1-based, 0: 0-based) */
-  int npf;        /* records whose A and B blocks are prefetched into L2 (0: none) */
-  int Ls[3];      /* entries per chunk in the CTA groups [0, slotn), [slotn, 2 slotn), [2 slotn, ...) */
-  int slotn;      /* CTA groups per length class (the SM count when the lengths differ) */
-};
-
 /* First entry of chunk c (0 <= c <= nchunks; S at the end) when CTA group b = c / W holds W chunks
    of Ls[class of b] entries. The host makes the three lengths equal (chunk c starts at c L), or, for
    a one-wave launch of several CTAs per SM, longer for the CTAs launched first on their SM and
@@ -174,26 +75,6 @@ __device__ __forceinline__ int chunk_first(const StackTask& tk, int W, int c) {
   const int Lb = (b < sn) ? tk.Ls[0] : ((b < 2 * sn) ? tk.Ls[1] : tk.Ls[2]);
   const long long f = (long long)W * (n0 * tk.Ls[0] + n1 * tk.Ls[1] + n2 * tk.Ls[2]) + (long long)w * Lb;
   return (int)min(f, (long long)tk.S);
-}
-
-/* Bulk prefetch into L2 of the A and B blocks of the first tk.npf parameter records, dealt round-robin
-   over the CTAs (record i to CTA i mod grid), so that every SM's copy unit issues a share. It reads only the caller's inputs (the raw stack and the pools), so a stack kernel
-   runs it before pdl_wait, while the grouping that precedes it in the stream still runs and the
-   pools would otherwise be fetched only at the first copy. A block's window is widened to 16-byte
-   boundaries (the bulk-copy granule); a widened window never leaves the block's page. */
-__device__ __forceinline__ void prefetch_block(const double* p, uint32_t bytes) {
-  const uint64_t s = (uint64_t)p, s0 = s & ~15ull, s1 = (s + bytes + 15ull) & ~15ull;
-  xs_tc::bulk_prefetch_l2((const void*)s0, (uint32_t)(s1 - s0));
-}
-__device__ __forceinline__ void prefetch_operands(const StackTask& tk) {
-  if (0 >= tk.npf) return;
-  const uint32_t abytes = (uint32_t)(tk.m * tk.k * sizeof(double)), bbytes = (uint32_t)(tk.k * tk.n * sizeof(double));
-  const int nthreads = (int)(gridDim.x * blockDim.x);
-  for (int i = (int)(blockIdx.x + gridDim.x * threadIdx.x); i < tk.npf; i += nthreads) {
-    const int* const e = tk.raw + (size_t)tk.rstride * i + tk.rbase;
-    prefetch_block(tk.a + (e[0] + tk.rshift), abytes);
-    prefetch_block(tk.b + (e[1] + tk.rshift), bbytes);
-  }
 }
 
 template <int MT, int NT>
@@ -1676,6 +1557,8 @@ int uni_staged_index(int m, int n, int k) {
 struct SmmPlan {
   int nsub_m, nsub_n, nsub, nchunks, L, W, ngroups;
   int Ls[3], slotn; /* chunk lengths per CTA length class (chunk_first) */
+  int tile; /* the tile kernel runs the stack, as tp says; then chunks are groups of their own (W = 1) */
+  xs_tile_plan_t tp;
   int no_combine; /* the stack kernel only: CTA-crossing pieces are combined by the caller */
   size_t off_keys_in, off_keys_tmp, off_keys_out, off_vals_in, off_vals_tmp, off_vals_out, off_seglist, off_pieces;
   size_t off_arrive, off_sort, total;
@@ -1719,46 +1602,70 @@ static int plan_nchunks(const SmmPlan& pl, int S) {
   return 2 * pl.W * pl.slotn + (int)((S - cap0 - cap1 + pl.Ls[2] - 1) / pl.Ls[2]);
 }
 
+/* Whether the tile kernel (smm_tile.cu) takes a stack: one without a tuned record, without a kernel staged for
+   its very shape (23^3, 30000: 59 us against 68) and not predicted for the FMA kernel, of at least 7e5
+   DMMA steps. The tile kernel beats the register kernel at every larger stack measured (32^3, 18640: 107 ->
+   91 us; 48^3, 4063: 87 -> 70); below, its teams hold a few entries each and their pieces cost more than
+   the staging saves (32x40x6, 4944: 35 -> 39 us; 45x44x5, 751: 21 -> 28). */
+static bool use_tile(int m, int n, int k, int S, const xs_smm_params_t* prm) {
+  const double steps = (double)S * ((m + 7) / 8) * ((n + 7) / 8) * ((k + 3) / 4);
+  return 0 != prm->tile && XS_KP_FMA != prm->kp && 0 != prm->kp && steps >= 7e5;
+}
+
 int plan_smm(int S, int m, int n, int k, const xs_smm_params_t* prm, SmmPlan* pl) {
-  const int mt = prm->mt, nt = prm->nt;
+  int mt = prm->mt, nt = prm->nt;
   double auto_skew = 0.0;
   if (mt < 1 || mt > 8 || nt < 1 || nt > 8) return -1; /* tiles beyond 4 fragments: staged kernels only */
   pl->no_combine = 0;
-  pl->nsub_m = ((m + 7) / 8 + mt - 1) / mt;
-  pl->nsub_n = ((n + 7) / 8 + nt - 1) / nt;
-  if (XS_KP_FMA == prm->kp) pl->nsub_m = pl->nsub_n = 1; /* the FMA lane grid covers the whole block */
-  pl->nsub = pl->nsub_m * pl->nsub_n;
-  pl->W = (prm->wpb >= 1 && prm->wpb <= 4) ? prm->wpb : 4;
-  if (0 == prm->generic && 4 < prm->wpb && nullptr != find_ws(m, n, k, prm->wpb) && (m + 7) / 8 == mt && (n + 7) / 8 == nt) {
-    pl->W = prm->wpb; /* warp-specialised kernel: wpb consumer warps, one chunk each */
+  pl->tile = (use_tile(m, n, k, S, prm) && 0 == xs_tile_plan(S, m, n, k, &pl->tp)) ? 1 : 0;
+  if (pl->tile) {
+    mt = pl->tp.mt;
+    nt = pl->tp.nt;
+    pl->nsub = pl->tp.T;
+    pl->nchunks = pl->ngroups = pl->tp.nchunks;
+    pl->nsub_n = pl->tp.nsub_n;
+    pl->nsub_m = pl->nsub / pl->nsub_n;
+    pl->L = pl->Ls[0] = pl->Ls[1] = pl->Ls[2] = pl->tp.L;
+    pl->slotn = 1 << 29;
+    pl->W = 1;
   }
-  if (0 < prm->chunk) pl->L = prm->chunk;
   else {
-    int occ = 0;
-    StackTask none = {};
-    none.m = m; /* the shape sizes the shared memory of runtime-shape kernels */
-    none.n = n;
-    none.k = k;
-    const launch_fn_t fn = find_launcher(m, n, k, prm);
-    if (cudaSuccess != fn(*pl, none, nullptr, nullptr, 0, &occ) || occ < 1) occ = 1;
-    const long resident = (long)occ * xs_sm_count();
-    const long L = ((long)S * pl->nsub + resident * pl->W - 1) / (resident * pl->W);
-    pl->L = (int)(L < 1 ? 1 : L);
-    auto_skew = (3 == occ && 1 == pl->nsub && S <= xs_stack_group_cluster_max()) ? chunk_skew() : 0.0;
-  }
-  pl->Ls[0] = pl->Ls[1] = pl->Ls[2] = pl->L;
-  pl->slotn = 1 << 29;
-  {
-    const int d = (int)(auto_skew * pl->L + 0.5);
-    if (0 < d && d < pl->L) { /* a one-wave launch of three CTAs per SM: the first-launched third of the
-                                 CTA groups takes L + d entries per chunk, the last third L - d */
-      pl->Ls[0] = pl->L + d;
-      pl->Ls[2] = pl->L - d;
-      pl->slotn = xs_sm_count();
+    pl->nsub_m = ((m + 7) / 8 + mt - 1) / mt;
+    pl->nsub_n = ((n + 7) / 8 + nt - 1) / nt;
+    if (XS_KP_FMA == prm->kp) pl->nsub_m = pl->nsub_n = 1; /* the FMA lane grid covers the whole block */
+    pl->nsub = pl->nsub_m * pl->nsub_n;
+    pl->W = (prm->wpb >= 1 && prm->wpb <= 4) ? prm->wpb : 4;
+    if (0 == prm->generic && 4 < prm->wpb && nullptr != find_ws(m, n, k, prm->wpb) && (m + 7) / 8 == mt && (n + 7) / 8 == nt) {
+      pl->W = prm->wpb; /* warp-specialised kernel: wpb consumer warps, one chunk each */
     }
+    if (0 < prm->chunk) pl->L = prm->chunk;
+    else {
+      int occ = 0;
+      StackTask none = {};
+      none.m = m; /* the shape sizes the shared memory of runtime-shape kernels */
+      none.n = n;
+      none.k = k;
+      const launch_fn_t fn = find_launcher(m, n, k, prm);
+      if (cudaSuccess != fn(*pl, none, nullptr, nullptr, 0, &occ) || occ < 1) occ = 1;
+      const long resident = (long)occ * xs_sm_count();
+      const long L = ((long)S * pl->nsub + resident * pl->W - 1) / (resident * pl->W);
+      pl->L = (int)(L < 1 ? 1 : L);
+      auto_skew = (3 == occ && 1 == pl->nsub && S <= xs_stack_group_cluster_max()) ? chunk_skew() : 0.0;
+    }
+    pl->Ls[0] = pl->Ls[1] = pl->Ls[2] = pl->L;
+    pl->slotn = 1 << 29;
+    {
+      const int d = (int)(auto_skew * pl->L + 0.5);
+      if (0 < d && d < pl->L) { /* a one-wave launch of three CTAs per SM: the first-launched third of the
+                                   CTA groups takes L + d entries per chunk, the last third L - d */
+        pl->Ls[0] = pl->L + d;
+        pl->Ls[2] = pl->L - d;
+        pl->slotn = xs_sm_count();
+      }
+    }
+    pl->nchunks = plan_nchunks(*pl, S);
+    pl->ngroups = (pl->nchunks + pl->W - 1) / pl->W;
   }
-  pl->nchunks = plan_nchunks(*pl, S);
-  pl->ngroups = (pl->nchunks + pl->W - 1) / pl->W;
   size_t off = 0;
   const size_t ks = align_up(sizeof(unsigned) * (size_t)S, 256), vs = align_up(sizeof(unsigned long long) * (size_t)S, 256);
   pl->off_keys_in = off;
@@ -1776,7 +1683,7 @@ int plan_smm(int S, int m, int n, int k, const xs_smm_params_t* prm, SmmPlan* pl
   pl->off_seglist = off;
   off = align_up(off + sizeof(int) * ((size_t)pl->ngroups + 1), 256);
   pl->off_pieces = off; /* two pieces per CTA group and sub-tile, one warp's accumulators each */
-  const int regs = (XS_KP_FMA == prm->kp) ? fma_piece_regs(m, n, k) : mt * nt * 2;
+  const int regs = (!pl->tile && XS_KP_FMA == prm->kp) ? fma_piece_regs(m, n, k) : mt * nt * 2;
   if (0 >= regs) return -1;
   off = align_up(off + sizeof(double) * (size_t)2 * pl->ngroups * pl->nsub * regs * 32, 256);
   pl->off_arrive = off; /* segment counters [ngroups][nsub], then first-level counters [2 ngroups][nsub] */
@@ -2011,6 +1918,9 @@ struct UniPart {
   int mt, nt; /* warp tile in 8 x 8 fragments */
   int nsub, nsub_n, L, ngroups;
   double item_cost;
+  int solo; /* runs in a launch of its own, as pl and prm say, not in the persistent kernel */
+  SmmPlan pl;
+  xs_smm_params_t prm;
 };
 
 /* Work items per resident CTA the plan aims for: enough for the queue to even out items of unequal
@@ -2061,6 +1971,15 @@ int uni_occupancy(void) {
   return occ_cached[dev];
 }
 
+/* Parts of at least this many DMMA steps with a staged kernel or the tile kernel, and parts of at least this many
+   entries with any kernel, get a launch of their own: they fill the device by themselves, and the persistent
+   kernel, whose register allocation every kernel in it shares, runs them at a half to a sixth of that
+   speed. 12 stacks of 186k triples (45x26x22, 42000 the largest) on B200: 1.11 ms in the persistent kernel
+   alone, 0.66 with the parts of 1.5e6 steps apart (0.41 of it the persistent kernel, in which 57000 of 13x22x9
+   and 48000 of 32x5x5 still ran), 0.47 with those apart too. */
+constexpr double kSoloSteps = 1.5e6;
+constexpr int kSoloEntries = 32768;
+
 /* Work decomposition of a batch for the unified kernel: stacks split into parts of at most
    xs_stack_group_max() entries; per part its kernel (the staged item function of its shape, or the
    register kernel of a tile class of at most 4 x 4 fragments) and a chunk length L chosen so that every
@@ -2091,6 +2010,12 @@ int plan_uni(const libxstream_b200_stack_t* st, int ns, UniPlan* up) {
       p.nsub_n = (0 <= sidx) ? 1 : (fn + p.nt - 1) / p.nt;
       p.nsub = (0 <= sidx) ? 1 : ((fm + p.mt - 1) / p.mt) * p.nsub_n;
       up->ntotal += p.S;
+      p.solo = 0;
+      if (0 != prm.tile && (((double)p.S * fm * fn * ((k + 3) / 4) >= kSoloSteps && (0 <= sidx || use_tile(m, n, k, p.S, &prm))) ||
+                             p.S >= kSoloEntries)) {
+        p.prm = prm;
+        p.solo = (0 == plan_smm(p.S, m, n, k, &p.prm, &p.pl)) ? 1 : 0;
+      }
     }
   }
   if (0 == up->nparts) return 0;
@@ -2098,12 +2023,14 @@ int plan_uni(const libxstream_b200_stack_t* st, int ns, UniPlan* up) {
   if (0 >= up->occ) return -1;
   /* cost units: DMMA instructions per entry per warp plus a fixed per-entry overhead */
   double total = 0;
+  int shared_parts = 0;
   for (int q = 0; q < up->nparts; ++q) {
     const UniPart& p = up->part[q];
-    total += (double)p.S * p.nsub * (p.mt * p.nt * ((st[p.stack].k + 3) / 4) + 8);
+    shared_parts += p.solo ? 0 : 1;
+    if (!p.solo) total += (double)p.S * p.nsub * (p.mt * p.nt * ((st[p.stack].k + 3) / 4) + 8);
   }
   const double per_cta = total / ((double)up->occ * xs_sm_count());
-  const double items = (1 == up->nparts) ? 1.0 : fmin(kUniItemsMax, fmax(kUniItemsMin, per_cta / kUniItemCost));
+  const double items = (1 == shared_parts) ? 1.0 : fmin(kUniItemsMax, fmax(kUniItemsMin, per_cta / kUniItemCost));
   const double target = per_cta / items;
   size_t off = 0, poff = 0, narrive = 0;
   up->ngroups_total = 0;
@@ -2117,15 +2044,23 @@ int plan_uni(const libxstream_b200_stack_t* st, int ns, UniPlan* up) {
     p.L = (int)L;
     const int nchunks = (int)((p.S + L - 1) / L);
     p.ngroups = (nchunks + kUniW - 1) / kUniW;
+    if (p.solo) {
+      p.ngroups = p.pl.ngroups;
+      p.nsub = p.pl.nsub;
+      p.mt = p.pl.tile ? p.pl.tp.mt : p.prm.mt;
+      p.nt = p.pl.tile ? p.pl.tp.nt : p.prm.nt;
+    }
+    const int regs = (p.solo && !p.pl.tile && XS_KP_FMA == p.prm.kp) ? fma_piece_regs(st[p.stack].m, st[p.stack].n, st[p.stack].k)
+                                                                      : p.mt * p.nt * 2;
     p.item_cost = (double)kUniW * L * per_entry;
     up->off_part[q] = off;
     off += (size_t)p.S;
     up->pieces_off[q] = poff;
-    poff += (size_t)2 * p.ngroups * p.nsub * (p.mt * p.nt * 2) * 32;
+    poff += (size_t)2 * p.ngroups * p.nsub * regs * 32;
     up->arrive_off[q] = narrive;
     narrive += (size_t)3 * p.ngroups * p.nsub;
     up->ngroups_total += p.ngroups;
-    up->nitems += p.ngroups * p.nsub;
+    if (!p.solo) up->nitems += p.ngroups * p.nsub;
     up->order[q] = q;
   }
   for (int a = 1; a < up->nparts; ++a) { /* heaviest items first (insertion sort, stable) */
@@ -2346,6 +2281,27 @@ static void set_prefetch(StackTask& tk, const int* dev_stack, int S, int format,
   tk.npf = (0 < per) ? (int)((budget / per < S) ? budget / per : S) : 0;
 }
 
+/* The plan's decomposition of a stack into chunks and warp tiles. */
+static void plan_task(const SmmPlan& pl, StackTask* tk) {
+  tk->L = pl.L;
+  tk->nchunks = pl.nchunks;
+  tk->ngroups = pl.ngroups;
+  tk->nsub_n = pl.nsub_n;
+  tk->nsub = pl.nsub;
+  tk->Ls[0] = pl.Ls[0];
+  tk->Ls[1] = pl.Ls[1];
+  tk->Ls[2] = pl.Ls[2];
+  tk->slotn = pl.slotn;
+}
+
+/* The stack kernel of one planned stack. */
+static int launch_planned(const SmmPlan& pl, const xs_smm_params_t& prm, const StackTask& tk, int* seglist, unsigned* err,
+  cudaStream_t s) {
+  if (pl.tile) return xs_tile_launch(&pl.tp, &tk, err, s);
+  const launch_fn_t fn = find_launcher(tk.m, tk.n, tk.k, &prm);
+  return (int)fn(pl, tk, seglist, err, s, nullptr);
+}
+
 int xs_launch_smm_f64_ex(const int* dev_stack, int S, int format, double alpha, const double* a, const double* b, double* c,
   int m, int n, int k, const xs_smm_params_t* prm, void* scratch, size_t scratch_bytes, void* stream) {
   SmmPlan pl;
@@ -2373,7 +2329,7 @@ int xs_launch_smm_f64_ex(const int* dev_stack, int S, int format, double alpha, 
   int* const arrive = (int*)(base + pl.off_arrive);
   void* prof = xs_profile_begin(s);
   const int r = xs_stack_group_ex(dev_stack, S, format, (unsigned)(m * n), keys_in, vals_in, keys_tmp, vals_tmp, keys_out,
-    vals_out, seglist, arrive, 3 * pl.ngroups * pl.nsub, pl.L * pl.W, sort_scratch, s);
+    vals_out, seglist, arrive, 3 * pl.ngroups * pl.nsub, pl.tile ? 0 : pl.L * pl.W, sort_scratch, s);
   if (0 != r) return r;
   xs_profile_end(prof, "sort", 0.0, 48.0 * S, s);
   StackTask tk = {};
@@ -2388,19 +2344,10 @@ int xs_launch_smm_f64_ex(const int* dev_stack, int S, int format, double alpha, 
   tk.m = m;
   tk.n = n;
   tk.k = k;
-  tk.L = pl.L;
-  tk.nchunks = pl.nchunks;
-  tk.ngroups = pl.ngroups;
-  tk.nsub_n = pl.nsub_n;
-  tk.nsub = pl.nsub;
   tk.arrive = arrive; /* CTA-crossing segments are combined inside the stack kernel */
-  tk.Ls[0] = pl.Ls[0];
-  tk.Ls[1] = pl.Ls[1];
-  tk.Ls[2] = pl.Ls[2];
-  tk.slotn = pl.slotn;
+  plan_task(pl, &tk);
   set_prefetch(tk, dev_stack, S, format, prefetch_budget());
-  const launch_fn_t fn = find_launcher(m, n, k, prm);
-  return (int)fn(pl, tk, seglist, xs_sort_error_flag(sort_scratch), s, nullptr);
+  return launch_planned(pl, *prm, tk, seglist, (unsigned*)xs_sort_error_flag(sort_scratch), s);
 }
 
 size_t xs_smm_batch_scratch_bytes(const libxstream_b200_stack_t* stacks, int nstacks) {
@@ -2492,6 +2439,15 @@ int xs_launch_smm_batch(const libxstream_b200_stack_t* st, int ns, void* scratch
     tk.m = d.m;
     tk.n = d.n;
     tk.k = d.k;
+    tk.sid = q;
+    set_prefetch(tk, d.dev_param_stack + 3 * (size_t)p.first, p.S, 0,
+      (long long)(pf_scale * 8.0 * d.k * (double)(d.m + d.n) * p.S));
+    if (p.solo) {
+      plan_task(p.pl, &tk);
+      r = launch_planned(p.pl, p.prm, tk, seglist, (unsigned*)xs_sort_error_flag(sort_scratch), s);
+      if (0 != r) return r;
+      continue;
+    }
     tk.L = p.L;
     tk.Ls[0] = tk.Ls[1] = tk.Ls[2] = p.L;
     tk.slotn = 1 << 29;
@@ -2501,15 +2457,13 @@ int xs_launch_smm_batch(const libxstream_b200_stack_t* st, int ns, void* scratch
     tk.nsub = p.nsub;
     tk.cls = (p.mt - 1) * 4 + (p.nt - 1);
     tk.kind = p.kind;
-    tk.sid = q;
     tk.item_begin = bt.nitems;
-    set_prefetch(tk, d.dev_param_stack + 3 * (size_t)p.first, p.S, 0,
-      (long long)(pf_scale * 8.0 * d.k * (double)(d.m + d.n) * p.S));
     bt.t[bt.ntasks++] = tk;
     bt.nitems += p.ngroups * p.nsub;
     flops += 2.0 * d.m * d.n * d.k * (double)p.S;
     bytes += 8.0 * p.S * ((double)d.m * d.k + (double)d.k * d.n + 2.0 * d.m * d.n);
   }
+  if (0 == bt.nitems) return 0;
   const int grid = max(1, min(bt.nitems, up.occ * xs_sm_count()));
   prof = xs_profile_begin(s);
   r = (int)pdl_launch(xs_smm_uni_kernel, grid, 32 * kUniW, kUniSmem, s, bt, seglist, xs_sort_queue_counter(sort_scratch, 0),

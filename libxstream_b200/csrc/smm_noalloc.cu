@@ -70,6 +70,7 @@ size_t libxstream_b200_process_scratch_bytes(int stack_size, int m, int n, int k
   xs_smm_params_t prm;
   if (0 >= stack_size || 0 >= m || 0 >= n || 0 >= k || EXIT_SUCCESS != xs_smm_ensure_init()) return 0;
   xs_params_lookup((int)dbcsr_type_real_8, m, n, k, stack_size, &prm);
+  prm.tile = 0;
   return xs_smm_f64_scratch_bytes(stack_size, m, n, k, &prm);
 }
 
@@ -93,6 +94,7 @@ int libxstream_b200_process_noalloc(const int* host_param_stack, const int* dev_
   result = xs_smm_ensure_init();
   if (EXIT_SUCCESS != result) return result;
   xs_params_lookup((int)datatype, m_max, n_max, k_max, stack_size, &prm);
+  prm.tile = 0; /* the tile kernel's pieces need more scratch than the array holds for stacks it took so far */
   nbytes = xs_smm_f64_scratch_bytes(stack_size, m_max, n_max, k_max, &prm);
   if (nbytes > XS_NOALLOC_SCRATCH_BYTES) {
     fprintf(stderr,

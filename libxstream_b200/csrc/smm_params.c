@@ -70,6 +70,7 @@ void xs_params_default(int m, int n, int k, int stack_size, xs_smm_params_t* out
   out->wpb = 4;
   out->sorted = 0;
   out->generic = 0;
+  out->tile = 1;
   { /* prefer a shape-specialised kernel with the same tiles (the first one listed) */
     int triples[3 * 8], i;
     const int nspec = xs_smm_f64_specialized(m, n, k, triples, 8);
@@ -161,6 +162,7 @@ int xs_params_set(int type, int m, int n, int k, const xs_smm_params_t* p, doubl
         r->k = k;
         r->gflops = gflops;
         r->p = *p;
+        r->p.tile = 0; /* tuned records run as they say */
         xs_sanitize(&r->p);
       }
       result = 0;
