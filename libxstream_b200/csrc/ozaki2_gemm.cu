@@ -21,7 +21,8 @@
  * moduli that give MB = 53 for this K (16 up to K = 2^17).
  *
  * Device layout: residue planes rA[q][M][Kp] and rB[q][N][Kp] (u8, K contiguous, zero padded),
- * exponents ea[M], eb[N], residues of C R[q][N][M] (u8, column-major per modulus).
+ * exponents ea[M], eb[N], residues of C R[q][N][Mp] (u8, column-major per modulus,
+ * Mp = M rounded up to 16).
  *
  * GEMM kernel: persistent, one CTA per SM, 10 warps, the pipeline of the scheme-1 kernel over work
  * units (modulus, 128 x 256 tile of C) taken modulus-major and strided by the grid: warp 0 streams
@@ -61,9 +62,9 @@ constexpr unsigned kModuli[kMaxMod] = {256, 255, 253, 251, 247, 241, 239, 233, 2
 
 struct Oz2Consts {
   unsigned mod[kMaxMod];
-  /* 32-bit residues (mod31): magic = floor(2^39 / m_i) + 1; c18 = 2^18 mod m_i, c36 = 2^36 mod m_i;
-     cneg = -2^54 mod m_i */
-  unsigned magic[kMaxMod], c18[kMaxMod], c36[kMaxMod], cneg[kMaxMod];
+  /* residues (residue_bytes16): bytes 2^0, 2^8, 2^16, 2^24 mod m_i; 2^32, 2^40, 2^48, -2^54 mod m_i;
+     magic = floor(2^32 / m_i) + 1 */
+  unsigned clo[kMaxMod], chi[kMaxMod], magic[kMaxMod];
   double phi, plo; /* P as a double-double */
   int nmod, mb;
   /* w_i = y_i / m_i as a 128-bit binary fraction (floor(2^128 y_i / m_i)), least significant word
@@ -73,14 +74,20 @@ struct Oz2Consts {
 
 /* --------------------------------------------------------------------------- preprocessing */
 
-/* Row maxima of the biased exponent, rows contiguous (element (r, k) at x[r + k*ld]); partial
-   maxima meet in emax[] (zeroed by the caller) by atomicMax. */
+/* Row maxima of the biased exponent, rows contiguous (element (r, k) at x[r + k*ld]), eight loads in
+   flight per thread; partial maxima meet in emax[] (zeroed by the caller) by atomicMax. */
 __global__ void xs_oz2_rowexp_rc(const double* __restrict__ x, long long ld, int R, int K, int kchunk, int* __restrict__ emax) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= R) return;
   const int k0 = blockIdx.y * kchunk, k1 = min(K, k0 + kchunk);
   int e = 0;
-  for (int k = k0; k < k1; ++k) e = max(e, biased_exp(x[r + (long long)k * ld]));
+  for (int k = k0; k < k1; k += 8) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = (k + u < k1) ? x[r + (long long)(k + u) * ld] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) e = max(e, biased_exp(v[u]));
+  }
   if (0 != e) atomicMax(emax + r, e);
 }
 
@@ -114,30 +121,36 @@ __device__ __forceinline__ unsigned mod31(unsigned x, unsigned m, unsigned magic
 }
 
 /* 16 consecutive k of one row as signed integers (-1)^s u, u < 2^53. A negative value is held as
-   u' = 2^54 - u (so that -u = u' + e (mod m) with e = -2^54 mod m), and u' <= 2^54 as 18-bit limbs
-   a0 + a1 2^18 + a2 2^36: its residue is that of x = a0 + a1 c18 + a2 c36 + s e < 2^27
-   (c = 2^18, 2^36 mod m), all 32-bit arithmetic. */
-struct Limbs16 {
-  unsigned a0[16], a1[16], a2[16], sg[16];
+   u' = 2^54 - u (so that -u = u' + e (mod m) with e = -2^54 mod m); the seven bytes of u' <= 2^54 and s as the
+   eighth one make the residue a dot product of eight bytes with 2^(8 i) mod m and e. */
+struct Bytes16 {
+  unsigned lo[16], hi[16];
 };
 
-__device__ __forceinline__ void limbs16(const double (&v)[16], int erow, int mb, Limbs16& L) {
+__device__ __forceinline__ void bytes16(const double (&v)[16], int erow, int mb, Bytes16& L) {
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
-    unsigned long long u = aligned_int(v[j], erow, mb, L.sg[j]);
-    if (L.sg[j]) u = (1ull << 54) - u;
-    L.a0[j] = (unsigned)u & 0x3ffffu;
-    L.a1[j] = (unsigned)(u >> 18) & 0x3ffffu;
-    L.a2[j] = (unsigned)(u >> 36);
+    unsigned sg;
+    unsigned long long u = aligned_int(v[j], erow, mb, sg);
+    if (sg) u = (1ull << 54) - u;
+    L.lo[j] = (unsigned)u;
+    L.hi[j] = (unsigned)(u >> 32) | (sg << 24);
   }
 }
 
-/* The 16 residues modulo m_i as bytes (k ascending). */
-__device__ __forceinline__ uint4 residue_bytes16(const Limbs16& L, const Oz2Consts& cs, int i) {
-  const unsigned m = cs.mod[i], mg = cs.magic[i], c1 = cs.c18[i], c2 = cs.c36[i], e = cs.cneg[i];
+/* The 16 residues modulo m_i as bytes (k ascending): two four-byte dot products give x < 7 * 255^2 + 255 <
+   2^19 with the value's residue; x * magic / 2^32 is x/m + x*e/2^32 with 0 < e <= 1, less than 2^-13 above
+   x/m, which is at most 1 - 1/m above an integer, so the high product is floor(x / m) exactly. This
+   pass is bound by these integer operations: with 18-bit limbs (three multiply-adds, a shifted high
+   product) 4096 x 4096 doubles took 141..153 us for 16 moduli, 125..138 with the dot products. */
+__device__ __forceinline__ uint4 residue_bytes16(const Bytes16& L, const Oz2Consts& cs, int i) {
+  const unsigned m = cs.mod[i], mg = cs.magic[i], cl = cs.clo[i], ch = cs.chi[i];
   unsigned r[16];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) r[j] = mod31(L.a0[j] + L.a1[j] * c1 + L.a2[j] * c2 + L.sg[j] * e, m, mg);
+  for (int j = 0; j < 16; ++j) {
+    const unsigned x = __dp4a(L.lo[j], cl, __dp4a(L.hi[j], ch, 0u));
+    r[j] = x - __umulhi(x, mg) * m;
+  }
   uint32_t w[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -169,8 +182,8 @@ __global__ void xs_oz2_res_kc(const double* __restrict__ x, long long ld, int R,
 #pragma unroll
     for (int j = 0; j < 16; ++j) v[j] = (k0 + j < K) ? row[k0 + j] : 0.0;
   }
-  Limbs16 L;
-  limbs16(v, emax[r], cs.mb, L);
+  Bytes16 L;
+  bytes16(v, emax[r], cs.mb, L);
   unsigned char* const dst = d + (long long)r * Kp + k0;
   const long long plane = (long long)R * Kp;
   for (int i = 0; i < cs.nmod; ++i) *reinterpret_cast<uint4*>(dst + i * plane) = residue_bytes16(L, cs, i);
@@ -190,8 +203,8 @@ __global__ void __launch_bounds__(256) xs_oz2_res_rc(const double* __restrict__ 
   double v[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) v[j] = (r < R && k0 + j < K) ? x[r + (long long)(k0 + j) * ld] : 0.0;
-  Limbs16 L;
-  limbs16(v, (r < R) ? emax[r] : 0, cs.mb, L);
+  Bytes16 L;
+  bytes16(v, (r < R) ? emax[r] : 0, cs.mb, L);
   const long long plane = (long long)R * Kp;
   /* write-out role: row wr of the tile, 16-byte chunk wc */
   const int wr = threadIdx.x >> 3, wc = threadIdx.x & 7;
@@ -224,12 +237,12 @@ __global__ void xs_oz2_scale_c(double* __restrict__ c, long long ldc, int M, int
 /* ------------------------------------------------------------------------------------ GEMM */
 
 struct Oz2GemmArgs {
-  int M, N, kb0, kb1; /* k-blocks [kb0, kb1) of 128 */
+  int M, N, Mp, kb0, kb1; /* rows of a residue plane of C (M rounded up to 16); k-blocks [kb0, kb1) of 128 */
   int nmod;
   int first; /* 1: the first k-chunk (residues are written, not accumulated) */
   unsigned mod[kMaxMod];
   unsigned magic[kMaxMod]; /* floor(2^39 / m_i) + 1 */
-  unsigned char* R; /* [nmod][N][M] */
+  unsigned char* R; /* [nmod][N][Mp] */
   unsigned* abort;
   unsigned* dev_err;
   long long wait_limit; /* bound of every pipeline wait, clock cycles */
@@ -354,26 +367,26 @@ __global__ void __launch_bounds__(kThreads, 1)
       tc_fence_after();
       const unsigned m = args.mod[q];
       const unsigned mg = args.magic[q];
-      unsigned char* const plane = args.R + (size_t)q * args.M * args.N;
+      unsigned char* const plane = args.R + (size_t)q * args.Mp * args.N;
       for (int c0 = cb; c0 < cb + kBN / 2; c0 += 32) {
         uint32_t v[32];
         tmem_ld32(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(buf * kBN + c0), v);
         tmem_ld_wait();
         if (rok) {
           const int ncol = min(32, args.N - (n0 + c0));
-          unsigned char* const dst = plane + row + (size_t)(n0 + c0) * args.M;
+          unsigned char* const dst = plane + row + (size_t)(n0 + c0) * args.Mp;
           if (!args.first) { /* a later k-chunk: add the residues so far */
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += (j < ncol) ? dst[(size_t)j * args.M] : 0u;
+            for (int j = 0; j < 32; ++j) v[j] += (j < ncol) ? dst[(size_t)j * args.Mp] : 0u;
           }
           if (32 == ncol) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) dst[(size_t)j * args.M] = (unsigned char)mod31(v[j], m, mg); /* < 2^31 */
+            for (int j = 0; j < 32; ++j) dst[(size_t)j * args.Mp] = (unsigned char)mod31(v[j], m, mg); /* < 2^31 */
           }
           else {
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
-              if (j < ncol) dst[(size_t)j * args.M] = (unsigned char)mod31(v[j], m, mg);
+              if (j < ncol) dst[(size_t)j * args.Mp] = (unsigned char)mod31(v[j], m, mg);
             }
           }
         }
@@ -410,30 +423,31 @@ __device__ __forceinline__ double crt_value(const uint32_t (&S)[4], const Oz2Con
 }
 
 /* C(i,j) = alpha * x * 2^E + beta * C(i,j), x the centred integer with residues R[.][j][i]. A thread
-   takes V consecutive rows i (one V-byte load per plane; V = 4 needs M % 4 == 0), grid rows take
-   columns j (strided when N exceeds the grid).
+   takes four consecutive rows i (one 4-byte load per plane; planes have Mp rows, a multiple of 16), grid
+   rows take columns j (strided when N exceeds the grid).
    x / P = frac(sum_i r_i w_i) is summed as a 128-bit binary fraction: the wrap-around modulo 2^128
    takes the fractional part and the two's-complement reading of the sum centres it to [-1/2, 1/2)
    (x in [-P/2, P/2)). With w_i rounded down to 2^-128 the fraction is off by less than
-   nmod * 255 * 2^-128 < 2^-115, i.e. x by less than 2^-115 P. */
-template <int V>
-__global__ void __launch_bounds__(256) xs_oz2_reconstruct(const unsigned char* __restrict__ R, int M, int N,
+   nmod * 255 * 2^-128 < 2^-115, i.e. x by less than 2^-115 P. The word columns are summed with wide integer
+   multiply-adds: the same sums as exact doubles on the FP64 pipe took twice the time (4096 x 4096 outputs,
+   16 moduli: 437 us against 223). */
+constexpr int kRecV = 4;
+__global__ void __launch_bounds__(256) xs_oz2_reconstruct(const unsigned char* __restrict__ R, int M, int N, int Mp,
   const int* __restrict__ ea, const int* __restrict__ eb, const __grid_constant__ Oz2Consts cs, double alpha, double beta,
   double* __restrict__ C, long long ldc) {
-  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * kRecV;
   if (i0 >= M) return;
-  const size_t plane = (size_t)M * N;
-  int ia[V];
+  const size_t plane = (size_t)Mp * N;
+  int ia[kRecV];
 #pragma unroll
-  for (int v = 0; v < V; ++v) ia[v] = (i0 + v < M) ? ea[i0 + v] : 0;
-  /* V residues per word; the next column's loads are in flight while this column is computed */
+  for (int v = 0; v < kRecV; ++v) ia[v] = (i0 + v < M) ? ea[i0 + v] : 0;
+  /* four residues per word; the next column's loads are in flight while this column is computed */
   unsigned res[kMaxMod], nxt[kMaxMod];
   auto load = [&](unsigned (&dst)[kMaxMod], int j) {
-    const size_t off = (size_t)j * M + i0;
+    const size_t off = (size_t)j * Mp + i0;
 #pragma unroll
     for (int q = 0; q < kMaxMod; ++q) {
-      if (4 == V) dst[q] = (q < cs.nmod) ? *reinterpret_cast<const unsigned*>(R + (size_t)q * plane + off) : 0u;
-      else dst[q] = (q < cs.nmod) ? R[(size_t)q * plane + off] : 0u;
+      dst[q] = (q < cs.nmod) ? *reinterpret_cast<const unsigned*>(R + (size_t)q * plane + off) : 0u;
     }
   };
   if (blockIdx.y < N) load(res, blockIdx.y);
@@ -442,7 +456,7 @@ __global__ void __launch_bounds__(256) xs_oz2_reconstruct(const unsigned char* _
     const int ib = eb[j];
     double* const cp = C + i0 + (long long)j * ldc;
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
+    for (int v = 0; v < kRecV; ++v) {
       /* sum_i r_i w_i column by column: word k of the product sums to < 20 * 2^8 * 2^32 < 2^45 in
          64 bits, so no carry moves until the columns are combined (modulo 2^128) at the end */
       unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
@@ -455,14 +469,12 @@ __global__ void __launch_bounds__(256) xs_oz2_reconstruct(const unsigned char* _
         }
       }
       uint32_t S[4];
-      unsigned long long t = acc[0];
-      S[0] = (uint32_t)t;
-      t = acc[1] + (t >> 32);
-      S[1] = (uint32_t)t;
-      t = acc[2] + (t >> 32);
-      S[2] = (uint32_t)t;
-      t = acc[3] + (t >> 32);
-      S[3] = (uint32_t)t;
+      unsigned long long t = 0ull;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        t = acc[w] + (t >> 32);
+        S[w] = (uint32_t)t;
+      }
       if (i0 + v < M) {
         const double val = (0 != ia[v] && 0 != ib) ? crt_value(S, cs, ia[v] + ib - 2150 + 2 * (53 - cs.mb)) : 0.0;
         cp[v] = (0.0 == beta) ? alpha * val : fma(alpha, val, beta * cp[v]);
@@ -563,10 +575,11 @@ int make_consts(int nmod, int K, Oz2Consts* cs) {
   for (int i = 0; i < nmod; ++i) {
     const unsigned m = kModuli[i];
     cs->mod[i] = m;
-    cs->magic[i] = (unsigned)((1ull << 39) / m + 1ull);
-    cs->c18[i] = (unsigned)((1ull << 18) % m);
-    cs->c36[i] = (unsigned)((1ull << 36) % m);
-    cs->cneg[i] = (unsigned)((m - (1ull << 54) % m) % m);
+    cs->magic[i] = (unsigned)((1ull << 32) / m + 1ull);
+    for (int b = 0; b < 4; ++b) {
+      cs->clo[i] |= (unsigned)((1ull << (8 * b)) % m) << (8 * b);
+      cs->chi[i] |= (unsigned)((3 == b) ? (m - (1ull << 54) % m) % m : (1ull << (32 + 8 * b)) % m) << (8 * b);
+    }
   }
   for (int i = 0; i < nmod; ++i) {
     const unsigned m = kModuli[i];
@@ -601,8 +614,9 @@ int default_nmod(int K) {
 int residue_operand(const double* x, long long ld, bool rows_contiguous, int R, int K, int Kp, const Oz2Consts& cs, int* emax,
   unsigned char* planes, cudaStream_t s) {
   if (rows_contiguous) {
-    const int kchunk = 256;
-    xs_oz2_rowexp_rc<<<dim3((R + 255) / 256, (K + kchunk - 1) / kchunk), 256, 0, s>>>(x, ld, R, K, kchunk, emax);
+    /* k ranges short enough that small operands fill the device too */
+    const int nrb = (R + 255) / 256, want = 4 * xs_sm_count() / nrb + 1, kchunk = max(16, min(256, (K + want - 1) / want));
+    xs_oz2_rowexp_rc<<<dim3(nrb, (K + kchunk - 1) / kchunk), 256, 0, s>>>(x, ld, R, K, kchunk, emax);
     xs_oz2_res_rc<<<dim3((R + kRcRows - 1) / kRcRows, (Kp + kRcK - 1) / kRcK), 256, 0, s>>>(x, ld, R, K, Kp, emax, cs, planes);
   }
   else {
@@ -627,7 +641,7 @@ int xs_ozaki2_default_moduli(int K) { return default_nmod(K > 0 ? K : 1); }
 size_t xs_ozaki2_gemm_scratch_bytes(int M, int N, int K, int nmod) {
   if (nmod <= 0) nmod = default_nmod(K > 0 ? K : 1);
   const size_t Kp = align_up((size_t)(K > 0 ? K : 1), 16);
-  return align_up((size_t)nmod * M * Kp, 1024) + align_up((size_t)nmod * N * Kp, 1024) + align_up((size_t)nmod * M * N, 1024) +
+  return align_up((size_t)nmod * M * Kp, 1024) + align_up((size_t)nmod * N * Kp, 1024) + align_up((size_t)nmod * align_up(M, 16) * N, 1024) +
          align_up(sizeof(int) * M, 256) + align_up(sizeof(int) * N, 256) + 256;
 }
 
@@ -656,7 +670,8 @@ int xs_ozaki2_gemm(char transa, char transb, int M, int N, int K, double alpha, 
   unsigned char* const rB = (unsigned char*)p;
   p += align_up((size_t)nmod * N * Kp, 1024);
   unsigned char* const rC = (unsigned char*)p;
-  p += align_up((size_t)nmod * M * N, 1024);
+  const int Mp = (int)align_up(M, 16);
+  p += align_up((size_t)nmod * Mp * N, 1024);
   int* const ea = (int*)p;
   p += align_up(sizeof(int) * M, 256);
   int* const eb = (int*)p;
@@ -675,10 +690,11 @@ int xs_ozaki2_gemm(char transa, char transb, int M, int N, int K, double alpha, 
   memset(&args, 0, sizeof(args));
   args.M = M;
   args.N = N;
+  args.Mp = Mp;
   args.nmod = nmod;
   for (int i = 0; i < nmod; ++i) {
     args.mod[i] = cs.mod[i];
-    args.magic[i] = cs.magic[i];
+    args.magic[i] = (unsigned)((1ull << 39) / cs.mod[i] + 1ull);
   }
   args.R = rC;
   args.abort = abort;
@@ -702,12 +718,9 @@ int xs_ozaki2_gemm(char transa, char transb, int M, int N, int K, double alpha, 
   }
   prof = xs_profile_begin(stream);
   const long long n = (long long)M * N;
-  const int V = (0 == M % 4) ? 4 : 1;
   /* about four waves of resident blocks; each thread walks its columns */
-  const int rgx = (M + 256 * V - 1) / (256 * V), rgy = max(1, min(N, min(65535, 12 * xs_sm_count() / rgx)));
-  const dim3 rgrid((unsigned)rgx, (unsigned)rgy);
-  if (4 == V) xs_oz2_reconstruct<4><<<rgrid, 256, 0, s>>>(rC, M, N, ea, eb, cs, alpha, beta, c, ldc);
-  else xs_oz2_reconstruct<1><<<rgrid, 256, 0, s>>>(rC, M, N, ea, eb, cs, alpha, beta, c, ldc);
+  const int rgx = (M + 256 * kRecV - 1) / (256 * kRecV), rgy = max(1, min(N, min(65535, 12 * xs_sm_count() / rgx)));
+  xs_oz2_reconstruct<<<dim3((unsigned)rgx, (unsigned)rgy), 256, 0, s>>>(rC, M, N, Mp, ea, eb, cs, alpha, beta, c, ldc);
   r = (int)cudaGetLastError();
   xs_profile_end(prof, "ozaki2_reconstruct", 0.0, (double)nmod * n + 16.0 * n, stream);
   return r;
