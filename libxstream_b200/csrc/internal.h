@@ -190,7 +190,7 @@ int xs_sort_launch_tiles(void);
 int xs_sort_tile_entries(int large);
 size_t xs_stack_sort_scratch_bytes(int S);
 size_t xs_stack_sort_scratch_bytes_batch(const xs_sort_batch_t* desc);
-/** Largest stack the one-cluster grouping kernel takes (entries). */
+/** Largest stack the one-cluster grouping kernel takes with four entries per thread. */
 int xs_stack_group_cluster_max(void);
 /** Largest single stack xs_stack_group takes in one launch (larger stacks are processed in parts). */
 int xs_stack_group_max(void);
@@ -202,7 +202,7 @@ int xs_stack_group(const int* dev_stack, int S, unsigned* k0, unsigned long long
   unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, void* sort_scratch, void* stream);
 /** As xs_stack_group, for either parameter format; also zeroes nzero ints at zero (nullptr: none).
     blk > 0: the C block size (blocks of the stack do not overlap), which spares the gcd statistics.
-    heavy > 0: in a single-pass grouping (stacks of at most 32768 entries over at most 2048 block
+    heavy > 0: in a single-pass grouping (stacks of at most 65536 entries over at most 2048 block
     positions), the C blocks with at least `heavy` entries come first, then the others, each class in
     offset order (entries of one block stay in stack order). */
 int xs_stack_group_ex(const int* dev_stack, int S, int format, unsigned blk, unsigned* k0, unsigned long long* v0, unsigned* k1,

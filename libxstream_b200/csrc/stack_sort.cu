@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kSortThreads) xs_stack_group_kernel(xs_sort_ba
 
 /* ------------------------------------------------------------------ one-cluster grouping (small stacks) */
 
-/* One-cluster grouping: 16 CTAs of 512 threads, 4 entries per thread (32768 entries at most). */
+/* One-cluster grouping: 16 CTAs of 512 threads, 4 entries per thread (32768 entries; see cluster_group_any). */
 constexpr int kClusterMax = 16;
 constexpr int kClThreads = 512;
 constexpr int kClWarps = kClThreads / 32;
@@ -544,7 +544,7 @@ constexpr int kClusterEntries = kClusterMax * kClThreads * kClE;
 constexpr size_t kClSmem = sizeof(unsigned short) * kClWarps * kRadix + sizeof(int) * kClusterMax * kRadix;
 
 
-/* Grouping of one stack of at most kClusterEntries entries by ONE thread-block cluster: a stable LSD
+/* Grouping of one stack of at most kClusterMax * kClThreads * E entries by ONE thread-block cluster: a stable LSD
    counting sort over the bucket ids of the c offsets, with the same per-digit order as
    xs_stack_group_kernel (stack order within a digit, hence the same output). Bucket ids: with blk > 0
    (the C block size: the blocks of one stack do not overlap, so distinct blocks lie at least blk
@@ -579,6 +579,11 @@ __global__ void __launch_bounds__(kClThreads) xs_stack_group_cluster_kernel(cons
     if (nullptr != stamps && 0 == threadIdx.x) stamps[rank * 8 + (slot)] = global_ns(); \
   } while (0)
   XS_CSTAMP(0);
+  /* launched with programmatic stream serialization: a stack kernel before this one in the stream lets it start
+     while its last CTAs still run; nothing is read or written before those are done. Only then may the stack
+     kernel after this one start (it reads the caller's stack and pools before its own wait). Hides the launch
+     from the call before it: 23x23x23, 30000, back to back 59.3 -> 55.9 us; 3000: 27.2 -> 23.9. */
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" :::);
   /* every CTA of the cluster must be running before another one writes into its shared memory: arrive
      now, wait before the first push (the stack loads overlap the barrier) */
@@ -861,13 +866,14 @@ int group_launch(const xs_sort_batch_t& desc0, unsigned* k0, unsigned long long*
     args, 0, s);
 }
 
-/* Launches the one-cluster grouping with ncta CTAs (a power of two <= kClusterMax). Returns
-   cudaErrorNotSupported, launching nothing, when the device cannot run a cluster of that size. */
+/* Launches the one-cluster grouping of E entries per thread with ncta CTAs (a power of two <= kClusterMax).
+   Returns cudaErrorNotSupported, launching nothing, when the device cannot run a cluster of that size. */
+template <int E>
 int cluster_group_launch(const int* stack, int S, int format, unsigned blk, unsigned* k0, unsigned long long* v0, unsigned* k1,
   unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, int* zero, int nzero, SortCtl* ctl, int ncta,
   int heavy, cudaStream_t s, unsigned long long* stamps = nullptr) {
   static int ok[XS_MAXDEV][kClusterMax + 1]; /* per device and cluster size: 0 unknown, 1 supported, -1 not */
-  auto kernel = xs_stack_group_cluster_kernel<kClE>;
+  auto kernel = xs_stack_group_cluster_kernel<E>;
   int* const okp = &ok[xs_device_slot()][ncta];
   const size_t smem = kClSmem;
   cudaLaunchConfig_t cfg = {};
@@ -875,11 +881,13 @@ int cluster_group_launch(const int* stack, int S, int format, unsigned blk, unsi
   cfg.blockDim = dim3(kClThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)ncta;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (0 == *okp) {
@@ -893,9 +901,25 @@ int cluster_group_launch(const int* stack, int S, int format, unsigned blk, unsi
     if (cudaSuccess != r) (void)cudaGetLastError(); /* not sticky: clear it */
   }
   if (0 > *okp) return (int)cudaErrorNotSupported;
+  cfg.numAttrs = 2;
   const unsigned blk_magic = (1u < blk) ? (unsigned)((1ull << 32) / blk) : 0u;
   return (int)cudaLaunchKernelEx(&cfg, kernel, stack, S, format, blk, k0, v0, k1, v1, kout, vout, seglist, zero, nzero, ctl, heavy,
     blk_magic, stamps);
+}
+
+/* Four entries per thread up to 32768 entries, eight up to 65536, where one cluster still beats the
+   cooperative kernel, which needs a memset before it and grid barriers (whole calls: 5x5x5, 60000: 46.2 ->
+   40.9 us; 13x13x13, 50000: 56.1 -> 49.8). With sixteen it does not (5x5x5, 100000: 55.2 -> 58.8 us). */
+constexpr int kClusterLarge = 2;
+int cluster_group_any(const int* stack, int S, int format, unsigned blk, unsigned* k0, unsigned long long* v0, unsigned* k1,
+  unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, int* zero, int nzero, SortCtl* ctl, int ncta,
+  int heavy, cudaStream_t s, unsigned long long* stamps = nullptr) {
+  if (S <= kClusterEntries) {
+    return cluster_group_launch<kClE>(stack, S, format, blk, k0, v0, k1, v1, kout, vout, seglist, zero, nzero, ctl, ncta, heavy, s,
+      stamps);
+  }
+  return cluster_group_launch<kClusterLarge * kClE>(stack, S, format, blk, k0, v0, k1, v1, kout, vout, seglist, zero, nzero, ctl,
+    ncta, heavy, s, stamps);
 }
 
 }  // namespace
@@ -946,10 +970,10 @@ int xs_stack_group(const int* dev_stack, int S, unsigned* k0, unsigned long long
 int xs_stack_group_ex(const int* dev_stack, int S, int format, unsigned blk, unsigned* k0, unsigned long long* v0, unsigned* k1,
   unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, int* zero, int nzero, int heavy,
   void* sort_scratch, void* stream) {
-  if (0 < S && S <= kClusterEntries) { /* one cluster of up to 16 CTAs */
+  if (0 < S && S <= kClusterLarge * kClusterEntries) { /* one cluster of up to 16 CTAs */
     int ncta = 1;
-    while (ncta * kClThreads * kClE < S) ncta <<= 1;
-    const int r = cluster_group_launch(dev_stack, S, format, blk, k0, v0, k1, v1, kout, vout, seglist, zero, nzero,
+    while (ncta < kClusterMax && ncta * kClThreads * kClE < S) ncta <<= 1;
+    const int r = cluster_group_any(dev_stack, S, format, blk, k0, v0, k1, v1, kout, vout, seglist, zero, nzero,
       (SortCtl*)sort_scratch, ncta, heavy, (cudaStream_t)stream);
     if (cudaErrorNotSupported != r) return r; /* else: the cooperative kernel below */
   }
@@ -1030,9 +1054,9 @@ int xs_stack_group_profile(const int* dev_stack, int S, unsigned blk, unsigned l
   d.blk[0] = blk;
   xs_sort_batch_t dp = d;
   int large = 0, ncta = 0;
-  if (0 < S && S <= kClusterEntries) {
+  if (0 < S && S <= kClusterLarge * kClusterEntries) {
     ncta = 1;
-    while (ncta * kClThreads * kClE < S) ncta <<= 1;
+    while (ncta < kClusterMax && ncta * kClThreads * kClE < S) ncta <<= 1;
   }
   const int grid = (0 < ncta) ? ncta : plan_tiles(&dp, &large);
   if (0 == grid || capacity < grid * 8) return -(int)cudaErrorInvalidValue;
@@ -1053,7 +1077,7 @@ int xs_stack_group_profile(const int* dev_stack, int S, unsigned blk, unsigned l
   unsigned long long* st = (unsigned long long*)p; p += 8 * sizeof(unsigned long long) * grid;
   int* seg = (int*)p; p += 256;
   p = (char*)(((uintptr_t)p + 255) & ~(uintptr_t)255);
-  int rc = (0 < ncta) ? cluster_group_launch(dev_stack, S, 0, blk, k0, v0, k1, v1, ko, vo, seg, nullptr, 0, (SortCtl*)p, ncta, 0, s, st)
+  int rc = (0 < ncta) ? cluster_group_any(dev_stack, S, 0, blk, k0, v0, k1, v1, ko, vo, seg, nullptr, 0, (SortCtl*)p, ncta, 0, s, st)
                       : cudaErrorNotSupported;
   if (cudaErrorNotSupported == rc) rc = group_launch(d, k0, v0, k1, v1, ko, vo, seg, p, s, st, 1);
   if (0 == rc) rc = (int)cudaMemcpyAsync(host_stamps, st, 8 * sizeof(unsigned long long) * grid, cudaMemcpyDeviceToHost, s);
