@@ -10,7 +10,7 @@
  *    rows8 x KP bytes (rows rounded up to 8 for A, 16 for B; KP = k rounded up to 32) made of core
  *    matrices of 8 rows x 16 bytes; exponents per block row / column.
  * 2. The stack is grouped by c (the plain path's grouping sort) and cut into chunks of L entries,
- *    one CTA per chunk (10 warps, 1 CTA per SM).
+ *    one CTA per chunk (18 warps, 1 CTA per SM).
  * 3. Per entry, warp 0 copies the entry's A and B digit tiles into a shared-memory stage with bulk
  *    copies. The B slices sit between zero slices, so the K-major operand starting at slice
  *    index d0 - sa spans B slices d0-sa .. d0-sa+W-1: one tcgen05.mma (M=64, N=W*n16, K=32) of A
@@ -19,10 +19,13 @@
  *    of diagonal d0+j (|sum| <= 8 * 127^2 * 64 < 2^23). Windows of W diagonals cover 0..cutoff;
  *    each (entry, window) owns one buffer of a tensor-memory ring, so the tensor cores run ahead of
  *    the epilogue.
- * 4. Warps 2-9 (epilogue): per (entry, window) they read the accumulator (M=64 layout: rows 16q..16q+15
- *    in lanes 32q..32q+15 of quarter q), combine the window's diagonals in FP64 with weights
- *    2^(-7j), scale by 2^(ea_i - 1029) * 2^(eb_j - 1029) * 2^(-7 d0) (exact powers of two) and add to
- *    the FP64 sum of the current segment (run of equal c) held in registers. A segment is written
+ * 4. Warps 2-17 (epilogue): per (entry, window) they read the accumulator (M=64 layout: rows 16q..16q+15
+ *    in lanes 32q..32q+15 of quarter q), combine the window's diagonals four at a time (two int32 pairs
+ *    D_j 2^7 + D_(j+1), then FP64), scale by 2^(ea_i - 1029) * 2^(eb_j - 1029) * 2^(-7 d) (exact powers
+ *    of two) and add to the FP64 sum of the current segment (run of equal c) held in registers. They
+ *    bound the kernel: eight warps that converted every diagonal by itself issued 2750 instructions per
+ *    entry each, 6 cycles apart (30000 entries of 64^3, 7 slices:
+ *    1.85 ms, 1.19 with sixteen and this recombination). A segment is written
  *    once: straight into C when it lies inside the chunk, else as a piece that the combine kernel
  *    adds up in chunk order (deterministic), as the plain path does.
  * Every mbarrier wait is bounded (per-call abort word, library device error word bit 2).
@@ -40,7 +43,7 @@ using namespace xs_oz;
 
 constexpr int kMaxSlices = 8;
 constexpr int kMaxWin = 16;
-constexpr int kEpiWarps = 8;
+constexpr int kEpiWarps = 16; /* four per tensor-memory lane quarter, a quarter of the columns each */
 constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kTmemCols = 512;
 constexpr unsigned kErrOzakiTimeout = 4u;
@@ -123,8 +126,13 @@ struct OzSmmArgs {
   long long wait_limit; /* bound of every pipeline wait, clock cycles */
 };
 
-__device__ __forceinline__ double pow2_or_zero(int e) { /* 2^(e - 1029) for a biased exponent e, 0 for e < 7 */
-  return (e >= 7) ? __longlong_as_double((long long)(e - 6) << 52) : 0.0;
+/* Blocks' rows and columns with a biased exponent below 7 count as zero. */
+constexpr int kMinExp = 7;
+/* 2^x, 0 and infinity included: exact over the normal range, rounded once below it. */
+__device__ __forceinline__ double pow2_wide(int x) {
+  if (x >= -1022 && x <= 1023) return __longlong_as_double((long long)(x + 1023) << 52);
+  const int y = max(-2044, min(x, 2046)), h = y >> 1;
+  return __longlong_as_double((long long)(h + 1023) << 52) * __longlong_as_double((long long)(y - h + 1023) << 52);
 }
 
 __device__ __forceinline__ void entry_blocks(const OzSmmArgs& g, unsigned long long v, int& ab, int& bb, bool& ok) {
@@ -255,17 +263,17 @@ __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_co
     }
   }
   else { /* epilogue: warps 2..9 */
-    const int ew = warp - 2, q = warp & 3, half = ew >> 2;
+    const int q = warp & 3, part = (warp - 2) >> 2;
     const int row = 16 * q + lane;
     const bool rok = (lane < 16) && (row < g.m);
-    const int nch = g.rowsB / 8, chalf = (nch + 1) / 2;
-    const int c_lo = half * chalf, c_hi = min(nch, c_lo + chalf);
+    const int nch = g.rowsB / 8, share = (nch + 3) / 4; /* 8-column chunks: at most two per warp */
+    const int c_lo = part * share, c_hi = min(nch, c_lo + share);
     const int mn = g.m * g.n;
     const bool headcross = (p0 > 0) && (g.keys[p0 - 1] == s_keys[0]);
     const bool tailcross = (p1 < g.S) && (s_keys[nent - 1] == g.keys[p1]);
-    double acc[4][8];
+    double acc[2][8];
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
+    for (int c = 0; c < 2; ++c)
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[c][j] = 0.0;
     int seg_start = p0;
@@ -286,7 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_co
         /* eight loads of C before their stores: one by one, each would wait for the one before (the compiler
            cannot know that they do not overlap) */
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < 2; ++c) {
           const int cc = c_lo + c;
           if (cc < c_hi) {
             double old[8];
@@ -300,7 +308,7 @@ __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_co
         }
       }
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
+      for (int c = 0; c < 2; ++c)
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[c][j] = 0.0;
     };
@@ -314,55 +322,42 @@ __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_co
       const int xs = e % kXSlots;
       if (!(ok = mbar_wait(&xfull[xs], (uint32_t)(e / kXSlots) & 1u, abort, 8u, g.wait_limit))) break;
       const int* const xe = xring + xs * 128;
-      const double rs = rok ? pow2_or_zero(xe[row]) : 0.0;
+      const int er = rok ? xe[row] : 0;
       for (int w = 0; w < g.nwin; ++w, ++grp) {
         const int buf = grp % g.nbuf, use = grp / g.nbuf;
         if (!(ok = mbar_wait(&accf[buf], (uint32_t)use & 1u, abort, 8u, g.wait_limit))) break;
         tc_fence_after();
         const OzWin& wn = g.win[w];
         const uint32_t tbase = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * g.bufcols);
-        const double rw = rs * __longlong_as_double((long long)(1023 - 7 * wn.d0) << 52);
-        /* two passes of up to two 8-column chunks: the window's diagonals are combined in FP64 with
-           weights 2^(-7 jb), then scaled and added to the segment sum */
+        /* up to four diagonals j0.. of a chunk at a time: pairs D_j 2^7 + D_(j+1) in int32 (|D| < 2^23), the two
+           pairs in FP64, then scaled and added to the segment sum */
+        for (int j0 = 0; j0 < wn.W; j0 += 4) {
+          const int left = wn.W - j0;
+          const int ew = er - 2058 - 7 * (wn.d0 + j0 + 1);
 #pragma unroll
-        for (int pass = 0; pass < 2; ++pass) {
-          double t[2][8];
+          for (int c = 0; c < 2; ++c) {
+            const int cc = c_lo + c;
+            if (cc >= c_hi) continue;
+            const uint32_t at = tbase + (uint32_t)(j0 * g.rowsB + cc * 8), step = (uint32_t)g.rowsB;
+            uint32_t v[4][8];
 #pragma unroll
-          for (int c = 0; c < 2; ++c)
+            for (int u = 1; u < 4; ++u)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) t[c][j] = 0.0;
-          double wd = 1.0;
-          for (int jb = 0; jb < wn.W; ++jb, wd *= 0.0078125) {
-            uint32_t v[2][8];
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const int cc = c_lo + 2 * pass + c;
-              if (cc < c_hi) tmem_ld8(tbase + (uint32_t)(jb * g.rowsB + cc * 8), v[c]);
-            }
+              for (int j = 0; j < 8; ++j) v[u][j] = 0u;
+            tmem_ld8(at, v[0]);
+            if (1 < left) tmem_ld8(at + step, v[1]);
+            if (2 < left) tmem_ld8(at + 2 * step, v[2]);
+            if (3 < left) tmem_ld8(at + 3 * step, v[3]);
+            const int4 e0 = *reinterpret_cast<const int4*>(xe + 64 + cc * 8), e1 = *reinterpret_cast<const int4*>(xe + 68 + cc * 8);
+            const int ec[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
             tmem_ld_wait();
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              if (c_lo + 2 * pass + c < c_hi) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) { /* exact int32 -> double: 2^52 + 2^31 + v, minus the offset */
-                  const double dv = __hiloint2double(0x43300000, (int)(v[c][j] ^ 0x80000000u)) - 4503601774854144.0;
-                  t[c][j] = fma(dv, wd, t[c][j]);
-                }
-              }
-            }
-          }
-          if (rok) {
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const int cc = c_lo + 2 * pass + c;
-              if (cc < c_hi) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  const int col = cc * 8 + j;
-                  const double cs = (col < g.n) ? pow2_or_zero(xe[64 + col]) : 0.0;
-                  acc[2 * pass + c][j] = fma(t[c][j], rw * cs, acc[2 * pass + c][j]);
-                }
-              }
+            for (int j = 0; j < 8; ++j) { /* exact int32 -> double: 2^52 + 2^31 + x, minus the offset */
+              const uint32_t x0 = (v[0][j] << 7) + v[1][j], x1 = (v[2][j] << 7) + v[3][j];
+              const double d0 = __hiloint2double(0x43300000, (int)(x0 ^ 0x80000000u)) - 4503601774854144.0;
+              const double d1 = __hiloint2double(0x43300000, (int)(x1 ^ 0x80000000u)) - 4503601774854144.0;
+              const double scale = (er >= kMinExp && ec[j] >= kMinExp) ? pow2_wide(ew + ec[j]) : 0.0;
+              acc[c][j] = fma(fma(d1, 0.00006103515625, d0), scale, acc[c][j]);
             }
           }
         }
