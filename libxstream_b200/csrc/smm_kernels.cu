@@ -2189,7 +2189,14 @@ __global__ void xs_norms_kernel(const double* __restrict__ mat, int nblks, const
   const double* const p = mat + offsets[blk];
   const int ne = nelems[blk];
   double s = 0.0;
-  for (int e = lane; e < ne; e += 32) s = fma(p[e], p[e], s);
+  /* eight loads in flight: one by one, a block of 22x22 took 15 trips to memory */
+  for (int e = lane; e < ne; e += 8 * 32) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = (e + 32 * u < ne) ? p[e + 32 * u] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s = fma(v[u], v[u], s);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (0 == lane) norms[blk] = (float)sqrt(s);
