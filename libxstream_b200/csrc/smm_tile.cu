@@ -560,21 +560,25 @@ int xs_tile_plan(int S, int m, int n, int k, xs_tile_plan_t* pl) {
   TileGeo geo;
   const int gk = 4 * pl->Q, ngrp = (k + gk - 1) / gk, cta_warps = c.T * c.nteam; /* panels are whole groups of indices */
   const int want = tile_warps(c.mt, c.nt), most = (want / cta_warps > 1) ? want / cta_warps : 1;
-  int ctas = most, grp = 0;
+  int ctas = most;
   pl->R = kStages;
-  for (int one = 1; one >= 0 && 0 == grp; --one) {
-    for (ctas = most; 0 == grp && ctas * cta_warps >= (one ? 8 : 1) && 0 < ctas; --ctas) {
-      const int budget = (227 * 1024 - 1536 * ctas) / ctas - slack;
-      for (grp = ngrp; grp > (one ? ngrp - 1 : 0); --grp) {
-        pl->npan = (ngrp + grp - 1) / grp;
-        pl->pk = (1 == pl->npan) ? k : (ngrp + pl->npan - 1) / pl->npan * gk;
-        if (make_geo(pl, m, n, &geo) * c.nteam <= budget) break;
-      }
-      if (grp == (one ? ngrp - 1 : 0)) grp = 0;
-      else break;
-    }
+  bool fits = false;
+  auto panels = [&](int npan) { /* whether a ring of entries in npan panels fits ctas times */
+    pl->npan = npan;
+    pl->pk = (1 == npan) ? k : (ngrp + npan - 1) / npan * gk;
+    pl->npan = (k + pl->pk - 1) / pl->pk;
+    return make_geo(pl, m, n, &geo) * c.nteam <= (227 * 1024 - 1536 * ctas) / ctas - slack;
+  };
+  for (int q = most; q > 0 && q * cta_warps >= 8 && !fits; --q) {
+    ctas = q;
+    fits = panels(1);
   }
-  if (0 == grp) return -1;
+  if (!fits) { /* as few panels as the longest that fits allows */
+    ctas = most;
+    if (!panels(ngrp)) return -1;
+    const int budget = ((227 * 1024 - 1536 * ctas) / ctas - slack) / c.nteam / kStages - 64, one = gk * 8 * (geo.a.ld + geo.b.ld);
+    for (int len = max(1, min(ngrp, budget / one)); !fits; --len) fits = panels((ngrp + len - 1) / len);
+  }
   pl->smem = (size_t)geo.region * c.nteam + slack;
   const void* const fn = (const void*)tile_kernel(c.mt, c.nt);
   int occ = 0;
