@@ -25,7 +25,7 @@
  *    of two) and add to the FP64 sum of the current segment (run of equal c) held in registers. They
  *    bound the kernel: eight warps that converted every diagonal by itself issued 2750 instructions per
  *    entry each, 6 cycles apart (30000 entries of 64^3, 7 slices:
- *    1.85 ms, 1.19 with sixteen and this recombination). A segment is written
+ *    1.85 ms, 1.19 with sixteen and this recombination, 0.85 with the scales as doubles). A segment is written
  *    once: straight into C when it lies inside the chunk, else as a piece that the combine kernel
  *    adds up in chunk order (deterministic), as the plain path does.
  * Every mbarrier wait is bounded (per-call abort word, library device error word bit 2).
@@ -53,45 +53,52 @@ constexpr int kXSlots = 8;      /* exponent ring: row exponents of A and column 
 
 /* ------------------------------------------------------------------------- pool slicing */
 
-/* Block blk, row r (< R) of K entries: element (r, kk) at x[blk*bs + r*rs + kk*cs]. Writes the digit
+/* Blocks' rows and columns with a biased exponent below 7 count as zero. */
+constexpr int kMinExp = 7;
+
+/* Block blk = blockIdx.x, row r (< R) of K entries: element (r, kk) at x[blk*bs + r*rs + kk*cs]. Writes the digit
    tiles d[blk][s][rows8][KP] (core matrices of 8 rows x 16 bytes: row group g at g*KP*8, k-chunk c
-   at c*128, row r%8 at 16*(r%8)) and the row exponents e[blk][64]. 64 threads per block. */
-__global__ void __launch_bounds__(128) xs_ozs_slice_pool(const double* __restrict__ x, int nblk, long long bs, int rs, int cs,
-  int R, int K, int KP, int rows8, int ns, unsigned char* __restrict__ d, int* __restrict__ e) {
-  const int blk = blockIdx.x * 2 + (threadIdx.x >> 6), r = threadIdx.x & 63;
-  if (blk >= nblk) return;
+   at c*128, row r%8 at 16*(r%8)) and the rows' scales w[blk][64] = 2^(emax - 1029 - shift), 0 for a row without a
+   large enough entry. One CTA per block, thread (r, c) takes the 16 entries of k-chunk c of row r: it reads them
+   once, all loads in flight, and the row's threads share their largest exponent in shared memory (64 threads per
+   block that walked whole rows twice took 93 us for 3750 blocks of 64x64). */
+__global__ void __launch_bounds__(256) xs_ozs_slice_pool(const double* __restrict__ x, long long bs, int rs, int cs, int R, int K,
+  int KP, int rows8, int ns, int shift, unsigned char* __restrict__ d, double* __restrict__ w) {
+  __shared__ int s_e[4][64];
+  const int blk = blockIdx.x, r = threadIdx.x & 63, c = threadIdx.x >> 6, nc = KP >> 4, k0 = 16 * c;
   const double* const xb = x + (long long)blk * bs;
+  double v[16];
   int emax = 0;
-  if (r < R) {
-    for (int kk = 0; kk < K; ++kk) emax = max(emax, biased_exp(xb[(long long)r * rs + (long long)kk * cs]));
-  }
-  e[(long long)blk * 64 + r] = emax;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = (r < R && k0 + j < K) ? xb[(long long)r * rs + (long long)(k0 + j) * cs] : 0.0;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) emax = max(emax, biased_exp(v[j]));
+  s_e[c][r] = emax;
+  __syncthreads();
+  for (int q = 0; q < nc; ++q) emax = max(emax, s_e[q][r]);
+  if (0 == c) w[(long long)blk * 64 + r] = (emax >= kMinExp) ? ldexp(1.0, emax - 1029 - shift) : 0.0;
   if (r >= rows8) return;
-  unsigned char* const out = d + (long long)blk * ns * rows8 * KP + (r >> 3) * (KP * 8) + (r & 7) * 16;
-  for (int k0 = 0; k0 < KP; k0 += 16) {
-    unsigned long long al[16];
-    unsigned sg[16];
+  unsigned char* const out = d + (long long)blk * ns * rows8 * KP + (r >> 3) * (KP * 8) + (r & 7) * 16 + c * 128;
+  unsigned long long al[16];
+  unsigned sg[16];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int kk = k0 + j;
-      const double v = (r < R && kk < K) ? xb[(long long)r * rs + (long long)kk * cs] : 0.0;
-      int be;
-      unsigned long long mt;
-      ieee_split(v, sg[j], be, mt);
-      const int sh = emax - be;
-      al[j] = (0 != mt && sh <= 52) ? (mt >> sh) : 0ull;
+  for (int j = 0; j < 16; ++j) {
+    int be;
+    unsigned long long mt;
+    ieee_split(v[j], sg[j], be, mt);
+    const int sh = emax - be;
+    al[j] = (0 != mt && sh <= 52) ? (mt >> sh) : 0ull;
+  }
+  for (int s = 0; s < ns; ++s) {
+    uint32_t q4[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      uint32_t u = 0;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) u |= ((uint32_t)(slice_digit(al[q * 4 + b], sg[q * 4 + b], s) & 0xFF)) << (8 * b);
+      q4[q] = u;
     }
-    for (int s = 0; s < ns; ++s) {
-      uint32_t w[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t v = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) v |= ((uint32_t)(slice_digit(al[q * 4 + b], sg[q * 4 + b], s) & 0xFF)) << (8 * b);
-        w[q] = v;
-      }
-      *reinterpret_cast<uint4*>(out + (long long)s * rows8 * KP + (k0 >> 4) * 128) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    *reinterpret_cast<uint4*>(out + (long long)s * rows8 * KP) = make_uint4(q4[0], q4[1], q4[2], q4[3]);
   }
 }
 
@@ -111,8 +118,8 @@ struct OzSmmArgs {
   long long mk, kn;
   const unsigned char* dA;
   const unsigned char* dB;
-  const int* eA;
-  const int* eB;
+  const double* wA; /* [na][64] row scales 2^(e - 1029) */
+  const double* wB; /* [nb][64] column scales 2^(e - 1029 - 7) */
   unsigned sliceA, sliceB;     /* bytes of one slice tile: rowsA*KP, rowsB*KP */
   unsigned stage_bytes, offB;  /* stage: A tiles at 0, B area (zero pads around the slices) at offB */
   int nstages;
@@ -125,15 +132,6 @@ struct OzSmmArgs {
   unsigned* dev_err;
   long long wait_limit; /* bound of every pipeline wait, clock cycles */
 };
-
-/* Blocks' rows and columns with a biased exponent below 7 count as zero. */
-constexpr int kMinExp = 7;
-/* 2^x, 0 and infinity included: exact over the normal range, rounded once below it. */
-__device__ __forceinline__ double pow2_wide(int x) {
-  if (x >= -1022 && x <= 1023) return __longlong_as_double((long long)(x + 1023) << 52);
-  const int y = max(-2044, min(x, 2046)), h = y >> 1;
-  return __longlong_as_double((long long)(h + 1023) << 52) * __longlong_as_double((long long)(y - h + 1023) << 52);
-}
 
 __device__ __forceinline__ void entry_blocks(const OzSmmArgs& g, unsigned long long v, int& ab, int& bb, bool& ok) {
   const long long ao = (long long)(unsigned)v - 1, bo = (long long)(unsigned)(v >> 32) - 1;
@@ -149,7 +147,7 @@ __device__ __forceinline__ void entry_blocks(const OzSmmArgs& g, unsigned long l
 __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_constant__ OzSmmArgs g) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* const smem = (unsigned char*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
-  int* const xring = (int*)(smem + (size_t)g.nstages * g.stage_bytes); /* [kXSlots][128]: eA row, eB col */
+  double* const xring = (double*)(smem + (size_t)g.nstages * g.stage_bytes); /* [kXSlots][128]: row, column scales */
   unsigned* const s_keys = (unsigned*)(xring + kXSlots * 128);           /* [kMaxChunk] */
   int2* const s_blk = (int2*)(s_keys + kMaxChunk);                       /* [kMaxChunk]: A, B block index */
   uint64_t* const bars = (uint64_t*)(s_blk + kMaxChunk);
@@ -212,12 +210,12 @@ __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_co
         const int stage = e % g.nstages;
         const uint32_t ph = (uint32_t)(e / g.nstages) & 1u;
         const int ab = s_blk[e].x, bb = s_blk[e].y;
-        { /* exponents of the entry's A rows and B columns into the exponent ring */
+        { /* scales of the entry's A rows and B columns into the scale ring */
           const int xs = e % kXSlots;
           if (!mbar_wait(&xempty[xs], ((uint32_t)(e / kXSlots) & 1u) ^ 1u, abort, 1u, g.wait_limit)) break;
-          mbar_arrive_expect_tx(&xfull[xs], 512);
-          bulk_load(xring + xs * 128, g.eA + (size_t)ab * 64, 256, &xfull[xs]);
-          bulk_load(xring + xs * 128 + 64, g.eB + (size_t)bb * 64, 256, &xfull[xs]);
+          mbar_arrive_expect_tx(&xfull[xs], 1024);
+          bulk_load(xring + xs * 128, g.wA + (size_t)ab * 64, 512, &xfull[xs]);
+          bulk_load(xring + xs * 128 + 64, g.wB + (size_t)bb * 64, 512, &xfull[xs]);
         }
         if (!mbar_wait(&empty[stage], ph ^ 1u, abort, 1u, g.wait_limit)) break;
         unsigned char* const st = smem + (size_t)stage * g.stage_bytes;
@@ -321,8 +319,8 @@ __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_co
       }
       const int xs = e % kXSlots;
       if (!(ok = mbar_wait(&xfull[xs], (uint32_t)(e / kXSlots) & 1u, abort, 8u, g.wait_limit))) break;
-      const int* const xe = xring + xs * 128;
-      const int er = rok ? xe[row] : 0;
+      const double* const xe = xring + xs * 128;
+      const double rs = rok ? xe[row] : 0.0;
       for (int w = 0; w < g.nwin; ++w, ++grp) {
         const int buf = grp % g.nbuf, use = grp / g.nbuf;
         if (!(ok = mbar_wait(&accf[buf], (uint32_t)use & 1u, abort, 8u, g.wait_limit))) break;
@@ -330,10 +328,10 @@ __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_co
         const OzWin& wn = g.win[w];
         const uint32_t tbase = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * g.bufcols);
         /* up to four diagonals j0.. of a chunk at a time: pairs D_j 2^7 + D_(j+1) in int32 (|D| < 2^23), the two
-           pairs in FP64, then scaled and added to the segment sum */
+           pairs in FP64, then scaled (the column scales hold the pairs' 2^-7) and added to the segment sum */
         for (int j0 = 0; j0 < wn.W; j0 += 4) {
           const int left = wn.W - j0;
-          const int ew = er - 2058 - 7 * (wn.d0 + j0 + 1);
+          const double rw = rs * __longlong_as_double((long long)(1023 - 7 * (wn.d0 + j0)) << 52);
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const int cc = c_lo + c;
@@ -348,16 +346,13 @@ __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_co
             if (1 < left) tmem_ld8(at + step, v[1]);
             if (2 < left) tmem_ld8(at + 2 * step, v[2]);
             if (3 < left) tmem_ld8(at + 3 * step, v[3]);
-            const int4 e0 = *reinterpret_cast<const int4*>(xe + 64 + cc * 8), e1 = *reinterpret_cast<const int4*>(xe + 68 + cc * 8);
-            const int ec[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 8; ++j) { /* exact int32 -> double: 2^52 + 2^31 + x, minus the offset */
               const uint32_t x0 = (v[0][j] << 7) + v[1][j], x1 = (v[2][j] << 7) + v[3][j];
               const double d0 = __hiloint2double(0x43300000, (int)(x0 ^ 0x80000000u)) - 4503601774854144.0;
               const double d1 = __hiloint2double(0x43300000, (int)(x1 ^ 0x80000000u)) - 4503601774854144.0;
-              const double scale = (er >= kMinExp && ec[j] >= kMinExp) ? pow2_wide(ew + ec[j]) : 0.0;
-              acc[c][j] = fma(fma(d1, 0.00006103515625, d0), scale, acc[c][j]);
+              acc[c][j] = fma(fma(d1, 0.00006103515625, d0), rw * xe[64 + cc * 8 + j], acc[c][j]);
             }
           }
         }
@@ -461,7 +456,7 @@ int plan_oz(int m, int n, int k, int ns, int cutoff, OzPlan* p) {
   p->nstages = (int)(budget / p->stage_bytes);
   if (p->nstages > 8) p->nstages = 8;
   if (p->nstages < 1) return -1;
-  p->smem = 128 + (size_t)p->nstages * p->stage_bytes + sizeof(int) * kXSlots * 128 + sizeof(unsigned) * kMaxChunk +
+  p->smem = 128 + (size_t)p->nstages * p->stage_bytes + sizeof(double) * kXSlots * 128 + sizeof(unsigned) * kMaxChunk +
             sizeof(int2) * kMaxChunk + 80 * sizeof(uint64_t);
   if (p->smem < 120 * 1024) p->smem = 120 * 1024; /* one CTA per SM: it owns all 512 TMEM columns */
   p->poolA = (size_t)ns * p->sliceA;
@@ -487,9 +482,9 @@ void layout_oz(const OzPlan& p, int S, int m, int n, int na, int nb, OzLayout* l
   l->dB = o;
   o = align_up(o + p.poolB * (size_t)nb, 256);
   l->eA = o;
-  o = align_up(o + sizeof(int) * 64 * (size_t)na, 256);
+  o = align_up(o + sizeof(double) * 64 * (size_t)na, 256);
   l->eB = o;
-  o = align_up(o + sizeof(int) * 64 * (size_t)nb, 256);
+  o = align_up(o + sizeof(double) * 64 * (size_t)nb, 256);
   const size_t ks = align_up(sizeof(unsigned) * (size_t)part, 256), vs = align_up(sizeof(unsigned long long) * (size_t)part, 256);
   l->keys0 = o;
   o += ks;
@@ -536,15 +531,15 @@ int xs_launch_smm_ozaki(const int* dev_stack, int S, int m, int n, int k, const 
   char* const base = (char*)scratch;
   unsigned char* const dA = (unsigned char*)(base + l.dA);
   unsigned char* const dB = (unsigned char*)(base + l.dB);
-  int* const eA = (int*)(base + l.eA);
-  int* const eB = (int*)(base + l.eB);
+  double* const wA = (double*)(base + l.eA);
+  double* const wB = (double*)(base + l.eB);
   unsigned* const abort = (unsigned*)(base + l.abort);
   int r = (int)cudaMemsetAsync(abort, 0, 256, s);
   if (0 != r) return r;
   void* prof = xs_profile_begin(stream);
   /* A block: element (i, kk) at i + kk*m; B block (k x n row-major): column j element kk at kk*n + j */
-  xs_ozs_slice_pool<<<(na + 1) / 2, 128, 0, s>>>(a, na, (long long)m * k, 1, m, m, k, p.KP, p.rowsA, p.ns, dA, eA);
-  xs_ozs_slice_pool<<<(nb + 1) / 2, 128, 0, s>>>(b, nb, (long long)k * n, 1, n, n, k, p.KP, p.rowsB, p.ns, dB, eB);
+  xs_ozs_slice_pool<<<na, 4 * p.KP, 0, s>>>(a, (long long)m * k, 1, m, m, k, p.KP, p.rowsA, p.ns, 0, dA, wA);
+  xs_ozs_slice_pool<<<nb, 4 * p.KP, 0, s>>>(b, (long long)k * n, 1, n, n, k, p.KP, p.rowsB, p.ns, 7, dB, wB);
   if (0 != (r = (int)cudaGetLastError())) return r;
   xs_profile_end(prof, "ozaki_slice_pools", 0.0, 8.0 * ((double)na * m * k + (double)nb * k * n), stream);
   if (0 != (r = xs_func_smem((const void*)xs_ozs_smm_kernel, p.smem))) return r;
@@ -581,8 +576,8 @@ int xs_launch_smm_ozaki(const int* dev_stack, int S, int m, int n, int k, const 
     g.kn = (long long)k * n;
     g.dA = dA;
     g.dB = dB;
-    g.eA = eA;
-    g.eB = eB;
+    g.wA = wA;
+    g.wB = wB;
     g.sliceA = p.sliceA;
     g.sliceB = p.sliceB;
     g.stage_bytes = p.stage_bytes;
