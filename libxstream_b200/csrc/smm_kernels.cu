@@ -1926,9 +1926,10 @@ struct UniPart {
 /* Work items per resident CTA the plan aims for: enough for the queue to even out items of unequal
    speed, few enough that an item's start (first copies in flight) and merge stay a small share. A
    batch of one part has items of equal speed: one per CTA. Otherwise one per kUniItemCost cost units
-   of work per CTA, between 6 and 16 (measured on B200: a 186k-triple mixed batch, 25k units per CTA,
-   is fastest with 6 items per CTA, a 2M-triple one, 275k units, with 12-24). */
-constexpr double kUniItemsMin = 6.0, kUniItemsMax = 16.0, kUniItemCost = 4000.0;
+   of work per CTA, between 2 and 16 (measured on B200: a 186k-triple mixed batch, 25k units per CTA,
+   is fastest with 6 items per CTA, a 2M-triple one, 275k units, with 12-24, and what other launches leave of a
+   batch, 3k units, with 2: 443 us for the whole call against 475 with 6 and 466 with 1). */
+constexpr double kUniItemsMin = 2.0, kUniItemsMax = 16.0, kUniItemCost = 4000.0;
 
 struct UniPlan {
   int nparts, ntotal, nitems, ngroups_total, occ;
@@ -1971,13 +1972,16 @@ int uni_occupancy(void) {
   return occ_cached[dev];
 }
 
-/* Parts of at least this many DMMA steps with a staged kernel or the tile kernel, and parts of at least this many
-   entries with any kernel, get a launch of their own: they fill the device by themselves, and the persistent
-   kernel, whose register allocation every kernel in it shares, runs them at a half to a sixth of that
-   speed. 12 stacks of 186k triples (45x26x22, 42000 the largest) on B200: 1.11 ms in the persistent kernel
-   alone, 0.66 with the parts of 1.5e6 steps apart (0.41 of it the persistent kernel, in which 57000 of 13x22x9
-   and 48000 of 32x5x5 still ran), 0.47 with those apart too. */
-constexpr double kSoloSteps = 1.5e6;
+/* Parts that get a launch of their own, because they fill the device by themselves and the persistent kernel,
+   whose register allocation every kernel in it shares, runs them slower:
+   - without a staged kernel: from kSoloSteps DMMA steps on the tile kernel, from kSoloEntries entries on with any
+     kernel (the persistent kernel runs the register kernel for them, at a half to a sixth of the speed). 12 stacks
+     of 186k triples (45x26x22, 42000 the largest) on B200: 1.11 ms in the persistent kernel alone, 0.66 with the
+     parts of 1.5e6 steps apart (0.41 of it the persistent kernel, in which 57000 of 13x22x9 and 48000 of 32x5x5
+     then ran), 0.47 with those apart too;
+   - with one: from kSoloStagedSteps on. 12 stacks of 2M triples, most of them staged: 2.21 -> 1.70 ms; the same
+     shapes at 186k triples are faster together (0.278 ms against 0.287 with parts of 1.5e6 steps apart). */
+constexpr double kSoloSteps = 1.5e6, kSoloStagedSteps = 4e6;
 constexpr int kSoloEntries = 32768;
 
 /* Work decomposition of a batch for the unified kernel: stacks split into parts of at most
@@ -2011,8 +2015,10 @@ int plan_uni(const libxstream_b200_stack_t* st, int ns, UniPlan* up) {
       p.nsub = (0 <= sidx) ? 1 : ((fm + p.mt - 1) / p.mt) * p.nsub_n;
       up->ntotal += p.S;
       p.solo = 0;
-      if (0 != prm.tile && (((double)p.S * fm * fn * ((k + 3) / 4) >= kSoloSteps && (0 <= sidx || use_tile(m, n, k, p.S, &prm))) ||
-                             p.S >= kSoloEntries)) {
+      const double work = (double)p.S * fm * fn * ((k + 3) / 4);
+      const bool large = (0 <= sidx) ? work >= kSoloStagedSteps
+                                     : (p.S >= kSoloEntries || (work >= kSoloSteps && use_tile(m, n, k, p.S, &prm)));
+      if (0 != prm.tile && large) {
         p.prm = prm;
         p.solo = (0 == plan_smm(p.S, m, n, k, &p.prm, &p.pl)) ? 1 : 0;
       }

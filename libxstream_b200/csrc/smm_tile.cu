@@ -539,6 +539,11 @@ extern "C" {
 int xs_tile_plan(int S, int m, int n, int k, xs_tile_plan_t* pl) {
   Choice c;
   if (S < 1 || m < 1 || n < 1 || k < 1 || !choose(m, n, k, &c)) return -1;
+  /* DMMA steps an entry must have for its staging to pay: few without padded operands, more with one or both
+     (200000 entries, register kernel -> this one: 13x22x9 196 -> 172 us, 14^3 157 -> 194; 13x32x22 332 -> 302,
+     48x9x9 350 -> 406; 32^3 875 -> 701, 16x32x32 464 -> 517, 48x48x5 557 -> 848) */
+  const int steps = ((m + 7) / 8) * ((n + 7) / 8) * ((k + 3) / 4), padded = (0 == m % 16 ? 1 : 0) + (0 == n % 16 ? 1 : 0);
+  if (steps < (0 == padded ? 18 : (1 == padded ? 48 : 128))) return -1;
   const int slack = 8 * (8 * (c.mt + c.nt) * 4 + 64); /* reads of padding rows and columns pass the last stage */
   int best = -1;
   for (int Q = 1; Q <= 4; Q *= 2) { /* the k distance with the fewest bank conflicts */
