@@ -76,7 +76,8 @@ __global__ void __launch_bounds__(kThreads, 3)
   double* const sB = smem + kStages * kATile;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
-  const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
+  const unsigned ntn = (unsigned)((N + kBN - 1) / kBN), bm = blockIdx.x / ntn;
+  const int m0 = (int)bm * kBM, n0 = (int)(blockIdx.x - bm * ntn) * kBN;
   const int nk = (K + kBK - 1) / kBK;
   double acc[4][4][2];
 #pragma unroll
@@ -139,7 +140,7 @@ cudaError_t launch(int M, int N, int K, double alpha, const double* A, int lda, 
   int ldc, cudaStream_t s) {
   const cudaError_t r = (cudaError_t)xs_func_smem((const void*)xs_dgemm_kernel<VEC>, smem_bytes());
   if (cudaSuccess != r) return r;
-  const dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM);
+  const unsigned grid = (unsigned)((N + kBN - 1) / kBN) * (unsigned)((M + kBM - 1) / kBM); /* M * N < 2^43 */
   xs_dgemm_kernel<VEC><<<grid, kThreads, smem_bytes(), s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
   return cudaGetLastError();
 }
