@@ -2370,8 +2370,8 @@ size_t xs_smm_batch_scratch_bytes(const libxstream_b200_stack_t* stacks, int nst
 }
 
 /* A batch of stacks: one grouping launch for up to XS_MAX_BATCH parts (more only when the parts
-   exceed the tiles one grouping launch takes), then one launch of the unified persistent kernel for
-   every part; no combine launch. */
+   exceed the tiles one grouping launch takes), then the parts that fill the device in launches of their
+   own, then one launch of the unified persistent kernel for all others, without a combine launch. */
 int xs_launch_smm_batch(const libxstream_b200_stack_t* st, int ns, void* scratch, size_t scratch_bytes, void* stream) {
   UniPlan up;
   cudaStream_t s = (cudaStream_t)stream;
