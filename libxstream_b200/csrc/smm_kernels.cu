@@ -1926,10 +1926,12 @@ struct UniPart {
 /* Work items per resident CTA the plan aims for: enough for the queue to even out items of unequal
    speed, few enough that an item's start (first copies in flight) and merge stay a small share. A
    batch of one part has items of equal speed: one per CTA. Otherwise one per kUniItemCost cost units
-   of work per CTA, between 2 and 16 (measured on B200: a 186k-triple mixed batch, 25k units per CTA,
-   is fastest with 6 items per CTA, a 2M-triple one, 275k units, with 12-24, and what other launches leave of a
-   batch, 3k units, with 2: 443 us for the whole call against 475 with 6 and 466 with 1). */
-constexpr double kUniItemsMin = 2.0, kUniItemsMax = 16.0, kUniItemCost = 4000.0;
+   of work per CTA, at most 16 and at least 6, or 2 beside parts launched alone (measured on B200: a
+   186k-triple mixed batch, 25k units per CTA, is fastest with 6 items per CTA, a 2M-triple one, 275k
+   units, with 12-24, and what other launches leave of a batch, 3k units, with 2: 443 us for the whole
+   call against 475 with 6 and 466 with 1. Without a part alone 2 lose: 43134 triples, 30879 of them
+   22x9x4, 253 us with 6 and 286 with 2, 37222 triples of up to 45x45x32 395 and 410). */
+constexpr double kUniItemsMin = 6.0, kUniItemsMinRest = 2.0, kUniItemsMax = 16.0, kUniItemCost = 4000.0;
 
 struct UniPlan {
   int nparts, ntotal, nitems, ngroups_total, occ;
@@ -2036,7 +2038,8 @@ int plan_uni(const libxstream_b200_stack_t* st, int ns, UniPlan* up) {
     if (!p.solo) total += (double)p.S * p.nsub * (p.mt * p.nt * ((st[p.stack].k + 3) / 4) + 8);
   }
   const double per_cta = total / ((double)up->occ * xs_sm_count());
-  const double items = (1 == shared_parts) ? 1.0 : fmin(kUniItemsMax, fmax(kUniItemsMin, per_cta / kUniItemCost));
+  const double least = (shared_parts < up->nparts) ? kUniItemsMinRest : kUniItemsMin;
+  const double items = (1 == shared_parts) ? 1.0 : fmin(kUniItemsMax, fmax(least, per_cta / kUniItemCost));
   const double target = per_cta / items;
   size_t off = 0, poff = 0, narrive = 0;
   up->ngroups_total = 0;
