@@ -32,6 +32,7 @@ using namespace xs_stack;
 constexpr int kMaxThreads = 320; /* 10 warps: a team of up to 10 warp tiles */
 constexpr int kStages = 2;
 constexpr int kMaxTeams = 8;
+constexpr int kSmemMax = 227 * 1024; /* shared memory of an SM that CTAs can use */
 constexpr int kFan = 8;     /* pieces per first-level sum of a long segment */
 constexpr unsigned kErrTileTimeout = 16u; /* device error word: a wait for block copies timed out (as the staged kernel) */
 
@@ -491,13 +492,14 @@ struct Choice {
    instruction and about 200 for a panel's wait, barrier and addresses. A lone warp with more than nine
    fragments loses to two warps (32^3: 167 us with one 4x4 tile, 135 with two 4x2). */
 bool choose(int m, int n, int k, Choice* c) {
-  const int fm = (m + 7) / 8, fn = (n + 7) / 8, ks = (k + 3) / 4;
+  const int fm = (m + 7) / 8, fn = (n + 7) / 8, ks = (k - 1) / 4 + 1;
   double best = -1.0;
   for (int mt = 1; mt <= 5; ++mt) {
     for (int nt = 1; nt <= 4; ++nt) {
       if (5 == mt && 2 != nt) continue;
-      const int T = ((fm + mt - 1) / mt) * ((fn + nt - 1) / nt);
-      if (T > kMaxThreads / 32 || 32 * T * tile_regs(mt, nt) > 65536) continue;
+      const long long tiles = (long long)((fm + mt - 1) / mt) * ((fn + nt - 1) / nt);
+      if (tiles > kMaxThreads / 32 || 32 * tiles * tile_regs(mt, nt) > 65536) continue;
+      const int T = (int)tiles;
       double cost = (double)T * (16.0 * mt * nt * ks + 200.0);
       if (1 == T && 9 < mt * nt) cost *= 1.25;
       if (best < 0.0 || cost < best) {
@@ -513,12 +515,15 @@ bool choose(int m, int n, int k, Choice* c) {
   return true;
 }
 
-/* Stage bytes of `cols` k indices. A bulk-copied window starts up to 8 bytes before the panel. */
-int stage_bytes(const OperandGeo& o, int rows, int cols) {
-  return o.padded ? (o.ld * cols * 8 + 15) / 16 * 16 : (rows * cols * 8 + 8 + 15) / 16 * 16;
+/* Stage bytes of `cols` k indices, in 64 bits: a whole block may have any k, and the bytes of a panel that does
+   not fit must not wrap to a size that does. A bulk-copied window starts up to 8 bytes before the panel. */
+long long stage_bytes(const OperandGeo& o, int rows, int cols) {
+  return o.padded ? (8ll * o.ld * cols + 15) / 16 * 16 : (8ll * rows * cols + 8 + 15) / 16 * 16;
 }
 
-int make_geo(const xs_tile_plan_t* pl, int m, int n, TileGeo* geo) {
+/* The launch geometry of a plan; returns the bytes of a team's ring. The sizes in geo are set only when the ring
+   fits an SM. */
+long long make_geo(const xs_tile_plan_t* pl, int m, int n, TileGeo* geo) {
   geo->T = pl->T;
   geo->nteam = pl->nteam;
   geo->Q = pl->Q;
@@ -527,23 +532,27 @@ int make_geo(const xs_tile_plan_t* pl, int m, int n, TileGeo* geo) {
   geo->R = pl->R;
   operand_geo(m, pl->Q, &geo->a);
   operand_geo(n, pl->Q, &geo->b);
-  geo->a.bytes = stage_bytes(geo->a, m, pl->pk);
-  geo->b.bytes = stage_bytes(geo->b, n, pl->pk);
-  geo->region = pl->R * (geo->a.bytes + geo->b.bytes);
-  return geo->region;
+  const long long ab = stage_bytes(geo->a, m, pl->pk), bb = stage_bytes(geo->b, n, pl->pk), region = pl->R * (ab + bb);
+  if (region <= kSmemMax) {
+    geo->a.bytes = (int)ab;
+    geo->b.bytes = (int)bb;
+    geo->region = (int)region;
+  }
+  return region;
 }
 
 }  // namespace
 
 extern "C" {
 
-int xs_tile_plan(int S, int m, int n, int k, xs_tile_plan_t* pl) {
+int xs_tile_geometry(int m, int n, int k, xs_tile_plan_t* pl) {
   Choice c;
-  if (S < 1 || m < 1 || n < 1 || k < 1 || !choose(m, n, k, &c)) return -1;
+  if (m < 1 || n < 1 || k < 1 || !choose(m, n, k, &c)) return -1;
   /* DMMA steps an entry must have for its staging to pay: few without padded operands, more with one or both
      (200000 entries, register kernel -> this one: 13x22x9 196 -> 172 us, 14^3 157 -> 194; 13x32x22 332 -> 302,
      48x9x9 350 -> 406; 32^3 875 -> 701, 16x32x32 464 -> 517, 48x48x5 557 -> 848) */
-  const int steps = ((m + 7) / 8) * ((n + 7) / 8) * ((k + 3) / 4), padded = (0 == m % 16 ? 1 : 0) + (0 == n % 16 ? 1 : 0);
+  const long long steps = (long long)((m + 7) / 8) * ((n + 7) / 8) * ((k - 1) / 4 + 1);
+  const int padded = (0 == m % 16 ? 1 : 0) + (0 == n % 16 ? 1 : 0);
   if (steps < (0 == padded ? 18 : (1 == padded ? 48 : 128))) return -1;
   const int slack = 8 * (8 * (c.mt + c.nt) * 4 + 64); /* reads of padding rows and columns pass the last stage */
   int best = -1;
@@ -564,7 +573,7 @@ int xs_tile_plan(int S, int m, int n, int k, xs_tile_plan_t* pl) {
   pl->nsub_n = ((n + 7) / 8 + c.nt - 1) / c.nt;
   /* as many CTAs per SM as the warps want, or down to 8 warps if that keeps entries in one panel */
   TileGeo geo;
-  const int gk = 4 * pl->Q, ngrp = (k + gk - 1) / gk, cta_warps = c.T * c.nteam; /* panels are whole groups of indices */
+  const int gk = 4 * pl->Q, ngrp = (k - 1) / gk + 1, cta_warps = c.T * c.nteam; /* panels are whole groups of indices */
   const int want = tile_warps(c.mt, c.nt), most = (want / cta_warps > 1) ? want / cta_warps : 1;
   int ctas = most;
   pl->R = kStages;
@@ -572,8 +581,8 @@ int xs_tile_plan(int S, int m, int n, int k, xs_tile_plan_t* pl) {
   auto panels = [&](int npan) { /* whether a ring of entries in npan panels fits ctas times */
     pl->npan = npan;
     pl->pk = (1 == npan) ? k : (ngrp + npan - 1) / npan * gk;
-    pl->npan = (k + pl->pk - 1) / pl->pk;
-    return make_geo(pl, m, n, &geo) * c.nteam <= (227 * 1024 - 1536 * ctas) / ctas - slack;
+    pl->npan = (k - 1) / pl->pk + 1;
+    return make_geo(pl, m, n, &geo) * c.nteam <= (kSmemMax - 1536 * ctas) / ctas - slack;
   };
   for (int q = most; q > 0 && q * cta_warps >= 8 && !fits; --q) {
     ctas = q;
@@ -582,16 +591,22 @@ int xs_tile_plan(int S, int m, int n, int k, xs_tile_plan_t* pl) {
   if (!fits) { /* as few panels as the longest that fits allows */
     ctas = most;
     if (!panels(ngrp)) return -1;
-    const int budget = ((227 * 1024 - 1536 * ctas) / ctas - slack) / c.nteam / kStages - 64, one = gk * 8 * (geo.a.ld + geo.b.ld);
+    const int budget = ((kSmemMax - 1536 * ctas) / ctas - slack) / c.nteam / kStages - 64, one = gk * 8 * (geo.a.ld + geo.b.ld);
     for (int len = max(1, min(ngrp, budget / one)); !fits; --len) fits = panels((ngrp + len - 1) / len);
   }
+  pl->ctas = ctas;
   pl->smem = (size_t)geo.region * c.nteam + slack;
-  const void* const fn = (const void*)tile_kernel(c.mt, c.nt);
+  return 0;
+}
+
+int xs_tile_plan(int S, int m, int n, int k, xs_tile_plan_t* pl) {
+  if (S < 1 || 0 != xs_tile_geometry(m, n, k, pl)) return -1;
+  const void* const fn = (const void*)tile_kernel(pl->mt, pl->nt);
   int occ = 0;
   if (0 != xs_func_smem(fn, pl->smem)) return -1;
-  if (cudaSuccess != cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 32 * c.T * c.nteam, pl->smem) || occ < 1) return -1;
-  if (occ > ctas) occ = ctas;
-  const long resident = (long)occ * xs_sm_count() * c.nteam;
+  if (cudaSuccess != cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 32 * pl->T * pl->nteam, pl->smem) || occ < 1) return -1;
+  if (occ > pl->ctas) occ = pl->ctas;
+  const long resident = (long)occ * xs_sm_count() * pl->nteam;
   pl->nchunks = (int)((S < resident) ? S : resident);
   pl->L = S / pl->nchunks;
   pl->rem = S - pl->L * pl->nchunks;

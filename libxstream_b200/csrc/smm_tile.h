@@ -14,10 +14,14 @@ typedef struct xs_tile_plan_t {
   int nsub_n;       /* warp tiles per row of the block */
   int Q;            /* distance of the k indices of a DMMA step */
   int pk, npan, R;  /* k indices per panel, panels per entry, stages of the ring */
+  int ctas;         /* CTAs per SM that the shared memory is cut for */
   int nchunks, L, rem; /* the first rem chunks hold L + 1 entries, the others L */
   size_t smem;
 } xs_tile_plan_t;
 
+/** The shape's part of a plan (all fields but nchunks, L, rem): host arithmetic only; nonzero when the tile
+    kernel does not take the shape. */
+int xs_tile_geometry(int m, int n, int k, xs_tile_plan_t* plan);
 /** Plans S entries of m x n x k; nonzero when the tile kernel does not take the shape. */
 int xs_tile_plan(int S, int m, int n, int k, xs_tile_plan_t* plan);
 /** Enqueues the kernel: task with operands, grouped entries, pieces (2 * nchunks * T tiles) and
