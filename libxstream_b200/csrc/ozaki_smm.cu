@@ -58,12 +58,12 @@ constexpr int kMinExp = 7;
 
 /* Block blk = blockIdx.x, row r (< R) of K entries: element (r, kk) at x[blk*bs + r*rs + kk*cs]. Writes the digit
    tiles d[blk][s][rows8][KP] (core matrices of 8 rows x 16 bytes: row group g at g*KP*8, k-chunk c
-   at c*128, row r%8 at 16*(r%8)) and the rows' scales w[blk][64] = 2^(emax - 1029 - shift), 0 for a row without a
+   at c*128, row r%8 at 16*(r%8)) and the rows' scales w[blk][64] = 2^(emax - 1029), 0 for a row without a
    large enough entry. One CTA per block, thread (r, c) takes the 16 entries of k-chunk c of row r: it reads them
    once, all loads in flight, and the row's threads share their largest exponent in shared memory (64 threads per
    block that walked whole rows twice took 93 us for 3750 blocks of 64x64). */
 __global__ void __launch_bounds__(256) xs_ozs_slice_pool(const double* __restrict__ x, long long bs, int rs, int cs, int R, int K,
-  int KP, int rows8, int ns, int shift, unsigned char* __restrict__ d, double* __restrict__ w) {
+  int KP, int rows8, int ns, unsigned char* __restrict__ d, double* __restrict__ w) {
   __shared__ int s_e[4][64];
   const int blk = blockIdx.x, r = threadIdx.x & 63, c = threadIdx.x >> 6, nc = KP >> 4, k0 = 16 * c;
   const double* const xb = x + (long long)blk * bs;
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) xs_ozs_slice_pool(const double* __restric
   s_e[c][r] = emax;
   __syncthreads();
   for (int q = 0; q < nc; ++q) emax = max(emax, s_e[q][r]);
-  if (0 == c) w[(long long)blk * 64 + r] = (emax >= kMinExp) ? ldexp(1.0, emax - 1029 - shift) : 0.0;
+  if (0 == c) w[(long long)blk * 64 + r] = (emax >= kMinExp) ? __longlong_as_double((long long)(emax - 6) << 52) : 0.0;
   if (r >= rows8) return;
   unsigned char* const out = d + (long long)blk * ns * rows8 * KP + (r >> 3) * (KP * 8) + (r & 7) * 16 + c * 128;
   unsigned long long al[16];
@@ -119,7 +119,7 @@ struct OzSmmArgs {
   const unsigned char* dA;
   const unsigned char* dB;
   const double* wA; /* [na][64] row scales 2^(e - 1029) */
-  const double* wB; /* [nb][64] column scales 2^(e - 1029 - 7) */
+  const double* wB; /* [nb][64] column scales 2^(e - 1029) */
   unsigned sliceA, sliceB;     /* bytes of one slice tile: rowsA*KP, rowsB*KP */
   unsigned stage_bytes, offB;  /* stage: A tiles at 0, B area (zero pads around the slices) at offB */
   int nstages;
@@ -327,11 +327,15 @@ __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_co
         tc_fence_after();
         const OzWin& wn = g.win[w];
         const uint32_t tbase = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * g.bufcols);
-        /* up to four diagonals j0.. of a chunk at a time: pairs D_j 2^7 + D_(j+1) in int32 (|D| < 2^23), the two
-           pairs in FP64, then scaled (the column scales hold the pairs' 2^-7) and added to the segment sum */
+        const double rw = rs * __longlong_as_double((long long)(1023 - 7 * wn.d0) << 52);
+        /* up to four diagonals j0.. of a chunk at a time: pairs 2^7 D_j + D_(j+1) in int32 (|D| < 2^23), read as
+           multiples of 2^(-7 j0 - 7), the two pairs in FP64, then scaled and added to the segment sum. The weight of
+           j0 is in the exponent that the integers are given, not in the row's scale, which it would carry below
+           the smallest double for rows of tiny entries whose products with large columns count */
         for (int j0 = 0; j0 < wn.W; j0 += 4) {
+          const int top = 0x42C00000 - ((7 * j0) << 20); /* high word of 2^(45 - 7 j0) */
+          const double offset = __hiloint2double(top, (int)0x80000000u);
           const int left = wn.W - j0;
-          const double rw = rs * __longlong_as_double((long long)(1023 - 7 * (wn.d0 + j0)) << 52);
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const int cc = c_lo + c;
@@ -348,11 +352,11 @@ __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_co
             if (3 < left) tmem_ld8(at + 3 * step, v[3]);
             tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 8; ++j) { /* exact int32 -> double: 2^52 + 2^31 + x, minus the offset */
+            for (int j = 0; j < 8; ++j) { /* exact int32 x -> double: 2^(45 - 7 j0) + (2^31 + x) 2^(-7 j0 - 7), minus the offset */
               const uint32_t x0 = (v[0][j] << 7) + v[1][j], x1 = (v[2][j] << 7) + v[3][j];
-              const double d0 = __hiloint2double(0x43300000, (int)(x0 ^ 0x80000000u)) - 4503601774854144.0;
-              const double d1 = __hiloint2double(0x43300000, (int)(x1 ^ 0x80000000u)) - 4503601774854144.0;
-              acc[c][j] = fma(fma(d1, 0.00006103515625, d0), rw * xe[64 + cc * 8 + j], acc[c][j]);
+              const double d0 = __hiloint2double(top, (int)(x0 ^ 0x80000000u)) - offset;
+              const double d1 = __hiloint2double(top, (int)(x1 ^ 0x80000000u)) - offset;
+              acc[c][j] = fma(fma(d1, 0x1p-14, d0), rw * xe[64 + cc * 8 + j], acc[c][j]);
             }
           }
         }
@@ -538,8 +542,8 @@ int xs_launch_smm_ozaki(const int* dev_stack, int S, int m, int n, int k, const 
   if (0 != r) return r;
   void* prof = xs_profile_begin(stream);
   /* A block: element (i, kk) at i + kk*m; B block (k x n row-major): column j element kk at kk*n + j */
-  xs_ozs_slice_pool<<<na, 4 * p.KP, 0, s>>>(a, (long long)m * k, 1, m, m, k, p.KP, p.rowsA, p.ns, 0, dA, wA);
-  xs_ozs_slice_pool<<<nb, 4 * p.KP, 0, s>>>(b, (long long)k * n, 1, n, n, k, p.KP, p.rowsB, p.ns, 7, dB, wB);
+  xs_ozs_slice_pool<<<na, 4 * p.KP, 0, s>>>(a, (long long)m * k, 1, m, m, k, p.KP, p.rowsA, p.ns, dA, wA);
+  xs_ozs_slice_pool<<<nb, 4 * p.KP, 0, s>>>(b, (long long)k * n, 1, n, n, k, p.KP, p.rowsB, p.ns, dB, wB);
   if (0 != (r = (int)cudaGetLastError())) return r;
   xs_profile_end(prof, "ozaki_slice_pools", 0.0, 8.0 * ((double)na * m * k + (double)nb * k * n), stream);
   if (0 != (r = xs_func_smem((const void*)xs_ozs_smm_kernel, p.smem))) return r;

@@ -93,3 +93,24 @@ def test_unsuitable_shapes_and_empty(acc):
     da = A.DevBuf.from_array(case.a, stream)
     assert A.process_ozaki(da, 0, 8, 8, 8, da, 4, da, 4, da, 7, 0, stream) == 0
     da.free()
+
+
+@pytest.mark.parametrize("n", [5, 16, 32])
+def test_rows_of_tiny_entries(acc, n):
+    """A row near the smallest normal number against a column near the largest: the scale of a late diagonal is
+    below the smallest double for the row alone, but not for the product. The only nonzero product is that of the
+    smallest entries, 2^-64, of their sixth and eighth digits; powers of two make it exact."""
+    A, stream = acc
+    m, k = 7, 9
+    a, b = np.zeros((k, m)), np.zeros((k, n))  # A column-major, B row-major
+    a[0], a[1] = 2.0**-987, 2.0**-1022
+    b[1], b[2] = 2.0**958, 2.0**1010
+    da, db, ds = (A.DevBuf.from_array(x, stream) for x in (a.ravel(), b.ravel(), np.ones(3, np.int32)))
+    dc = A.DevBuf(8 * m * n)
+    dc.zero(stream)
+    assert A.process_ozaki(ds, 1, m, n, k, da, 1, db, 1, dc, 8, 0, stream) == 0
+    got = dc.download(np.zeros(m * n), stream)
+    stream.sync()
+    assert np.array_equal(got, np.full(m * n, 2.0**-64))
+    for x in (da, db, ds, dc):
+        x.free()
