@@ -1602,14 +1602,24 @@ static int plan_nchunks(const SmmPlan& pl, int S) {
   return 2 * pl.W * pl.slotn + (int)((S - cap0 - cap1 + pl.Ls[2] - 1) / pl.Ls[2]);
 }
 
-/* Whether the tile kernel (smm_tile.cu) takes a stack: one without a tuned record, without a kernel staged for
+/* Whether the tile kernel (smm_tile.cu) may take a stack: one without a tuned record, without a kernel staged for
    its very shape (23^3, 30000: 59 us against 68) and not predicted for the FMA kernel, of at least 7e5
-   DMMA steps. The tile kernel beats the register kernel at every larger stack measured (32^3, 18640: 107 ->
-   91 us; 48^3, 4063: 87 -> 70); below, its teams hold a few entries each and their pieces cost more than
-   the staging saves (32x40x6, 4944: 35 -> 39 us; 45x44x5, 751: 21 -> 28). */
+   DMMA steps. Below, its teams hold a few entries each and their pieces cost more than the staging saves
+   (32x40x6, 4944: 35 -> 39 us; 45x44x5, 751: 21 -> 28); above, it beats the register kernel (32^3, 18640: 107 ->
+   91 us; 48^3, 4063: 87 -> 70) but for the shapes that xs_tile_geometry refuses. */
 static bool use_tile(int m, int n, int k, int S, const xs_smm_params_t* prm) {
   const double steps = (double)S * ((m + 7) / 8) * ((n + 7) / 8) * ((k + 3) / 4);
   return 0 != prm->tile && XS_KP_FMA != prm->kp && 0 != prm->kp && steps >= 7e5;
+}
+
+static bool spec_listed(int m, int n, int k, const xs_smm_params_t* prm);
+
+/* The tile kernel's plan of a stack, if it takes it. Teams of 4 x 4 tiles are eight warps per SM, which need five
+   entries each to win over a register kernel compiled for the very shape (64^3 in uniform C blocks: 832 entries
+   40 us against 45, 1173: 48 against 54, 1465: 57 against 59; 1500: 63 against 62; 2930: 98 against 94). */
+static bool plan_tile(int S, int m, int n, int k, const xs_smm_params_t* prm, xs_tile_plan_t* tp) {
+  if (!use_tile(m, n, k, S, prm) || 0 != xs_tile_plan(S, m, n, k, tp)) return false;
+  return 12 >= tp->mt * tp->nt || !spec_listed(m, n, k, prm) || S >= 5l * tp->ctas * tp->nteam * xs_sm_count();
 }
 
 int plan_smm(int S, int m, int n, int k, const xs_smm_params_t* prm, SmmPlan* pl) {
@@ -1617,7 +1627,7 @@ int plan_smm(int S, int m, int n, int k, const xs_smm_params_t* prm, SmmPlan* pl
   double auto_skew = 0.0;
   if (mt < 1 || mt > 8 || nt < 1 || nt > 8) return -1; /* tiles beyond 4 fragments: staged kernels only */
   pl->no_combine = 0;
-  pl->tile = (use_tile(m, n, k, S, prm) && 0 == xs_tile_plan(S, m, n, k, &pl->tp)) ? 1 : 0;
+  pl->tile = plan_tile(S, m, n, k, prm, &pl->tp) ? 1 : 0;
   if (pl->tile) {
     mt = pl->tp.mt;
     nt = pl->tp.nt;
@@ -1854,6 +1864,13 @@ static const SpecEntry spec_table[] = {
   XS_SPEC(4, 1, 1), XS_SPEC(5, 1, 2), XS_SPEC(8, 1, 2), XS_SPEC(9, 2, 3), XS_SPEC(16, 2, 2), XS_SPEC(16, 2, 4),
   XS_SPEC(32, 4, 2), XS_SPEC(32, 4, 4), XS_SPEC(45, 3, 2), XS_SPEC(45, 3, 4), XS_SPEC(64, 4, 2), XS_SPEC(64, 4, 4),
 };
+
+static bool spec_listed(int m, int n, int k, const xs_smm_params_t* prm) {
+  for (const SpecEntry& e : spec_table) {
+    if (e.m == m && e.n == n && e.k == k && e.mt == prm->mt && e.nt == prm->nt && e.kp == prm->kp) return 0 == prm->generic;
+  }
+  return false;
+}
 
 /* Shapes with a staged kernel: it runs whenever the warp tile covers the whole C block (any kp),
    unless the runtime-shape kernel is forced (generic). Each was measured against the register

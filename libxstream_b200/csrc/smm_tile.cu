@@ -484,13 +484,17 @@ void operand_geo(int rows, int Q, OperandGeo* o) {
   o->ld = o->padded ? rows + ((1 == Q) ? 4 : 2) : rows;
 }
 
+int teams_per_cta(int T) { return (T >= 4) ? 1 : 4 / T; }
+
 struct Choice {
   int mt, nt, T, nteam;
 };
 
 /* Warp tiles of an m x n block: the least time of all warps for one entry, 16 cycles per DMMA
    instruction and about 200 for a panel's wait, barrier and addresses. A lone warp with more than nine
-   fragments loses to two warps (32^3: 167 us with one 4x4 tile, 135 with two 4x2). */
+   fragments loses to two warps (32^3: 167 us with one 4x4 tile, 135 with two 4x2). Tiles that leave an SM
+   fewer than eight warps do not keep its FP64 pipe busy (one team of seven 1x4 tiles, 54x29x73, 9400 entries:
+   232 us against the register kernel's 189; now two of 4x4: 150). */
 bool choose(int m, int n, int k, Choice* c) {
   const int fm = (m + 7) / 8, fn = (n + 7) / 8, ks = (k - 1) / 4 + 1;
   double best = -1.0;
@@ -502,6 +506,8 @@ bool choose(int m, int n, int k, Choice* c) {
       const int T = (int)tiles;
       double cost = (double)T * (16.0 * mt * nt * ks + 200.0);
       if (1 == T && 9 < mt * nt) cost *= 1.25;
+      const int cta_warps = T * teams_per_cta(T), warps = cta_warps * max(1, tile_warps(mt, nt) / cta_warps);
+      if (8 > warps) cost *= 8.0 / warps;
       if (best < 0.0 || cost < best) {
         best = cost;
         c->mt = mt;
@@ -511,7 +517,7 @@ bool choose(int m, int n, int k, Choice* c) {
     }
   }
   if (best < 0.0) return false;
-  c->nteam = (c->T >= 4) ? 1 : 4 / c->T;
+  c->nteam = teams_per_cta(c->T);
   return true;
 }
 
@@ -595,6 +601,17 @@ int xs_tile_geometry(int m, int n, int k, xs_tile_plan_t* pl) {
     for (int len = max(1, min(ngrp, budget / one)); !fits; --len) fits = panels((ngrp + len - 1) / len);
   }
   pl->ctas = ctas;
+  /* DMMA instructions of a warp in a panel: they have to pay for the panel's wait, the team's barrier and, where
+     columns are padded, the copies that the team issues itself. Over 1230 stacks (all shapes up to 80, 7e5 to 5e6
+     steps) these lines leave out what was up to 1.4 times slower than the register kernel and, in the mean, as fast:
+     - panels of one or two DMMA steps (k <= 8) without padding only (32x76x5, 12502 entries: register kernel 65 us,
+       this one 83), with a second team beside them (77x64x7, 6252: 63, 79), and of at least 8 or 18 instructions
+       (7x72x7, 88890: 153, 178; 46x13x5, 192109: 228, 256; but 23x22x5, 88890: 99, 93);
+     - padded columns: never for a lone warp (16x32x64, 6252: 45, 52), and for a team of two in short entries only
+       from 25 instructions on (9x48x13, 33335: 86, 94; but 48x45x9, 46298: 251, 230). */
+  const int psteps = (min(pl->pk, k) - 1) / 4 + 1, instr = c.mt * c.nt * psteps;
+  if (2 >= psteps && (0 < padded || 1 == ctas * c.nteam || instr < (1 == psteps ? 8 : 18))) return -1;
+  if (0 < padded && (1 == c.T || (2 == c.T && 1 == pl->npan && instr < 25))) return -1;
   pl->smem = (size_t)geo.region * c.nteam + slack;
   return 0;
 }
