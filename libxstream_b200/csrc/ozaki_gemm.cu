@@ -50,10 +50,11 @@ using namespace xs_tc;
 using namespace xs_oz;
 
 constexpr int kBM = 128, kBN = 64, kBK = 32;
-constexpr int kSliceA = kBM * kBK, kSliceB = kBN * kBK; /* bytes of one slice of a panel */
 constexpr int kMaxSlices = 8;
 constexpr int kMaxDiag = 512 / kBN;       /* diagonals in tensor memory at a time */
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 9;
+constexpr int kStageBytes = 36 * 1024;    /* k blocks share a stage as long as it does not pass this size */
+constexpr int kRegOps = 4;
 constexpr int kMaxOps = 3 * kMaxSlices;   /* MMAs per k block */
 constexpr int kKChunkBlocks = 16384 / kBK; /* k blocks per launch: keeps every diagonal's int32 sum exact */
 constexpr int kEpiWarps = 8;
@@ -163,15 +164,19 @@ __global__ void xs_oz_scale_c(double* __restrict__ c, long long ldc, int M, int 
 
 /* ------------------------------------------------------------------------------ GEMM */
 
-/* One MMA of a k block: A slice sa against w B slices from sb on, into the columns of diagonal col; acc = 0
-   writes them, 1 adds to them. */
-struct OzOp {
-  unsigned char sa, sb, w, col, acc;
+/* One MMA of a k block: an A slice against adjacent B slices, into the columns of the first pair's diagonal. As the
+   issuing thread needs it, so that an MMA costs it one 16-byte read and a few additions. */
+struct alignas(16) OzOp {
+  uint32_t a, b;  /* offset of the A slice, of the first B slice in the k block, / 16 */
+  uint32_t d;     /* tensor-memory column; bit 31: add to the columns, else write them */
+  uint32_t idesc; /* instruction descriptor */
 };
 
 struct OzGemmArgs {
   int M, N, kb0, kb1, KB; /* k blocks [kb0, kb1) of KB */
   int ns, nstages;
+  int rows, cols;         /* of a digit panel of A, of B */
+  int kps;                /* k blocks per stage */
   int ndiag, eshift;      /* diagonals of the launch, -2058 - 7 d of the first */
   int first;              /* 1: this launch applies beta to C, later ones add to it */
   double alpha, beta;
@@ -188,9 +193,10 @@ struct OzGemmArgs {
   OzOp op[2][kMaxOps];
 };
 
-/* Shared memory: 128 bytes of alignment slack, the ring, its barriers, the tensor-memory address. */
-__host__ __device__ constexpr size_t oz_gemm_smem(int ns, int stages) {
-  return 128 + (size_t)stages * ns * (kSliceA + kSliceB) + (2 * kMaxStages + 2) * sizeof(uint64_t) + 16;
+/* Shared memory: 128 bytes of alignment slack, the ring, its barriers, the tensor-memory address; and what the MMAs, which
+   take 128 rows, read past the last slice of a panel with fewer (for rows of C that there are not). */
+size_t oz_gemm_smem(const OzGemmArgs& g) {
+  return 128 + (size_t)g.nstages * g.kps * g.ns * (g.rows + g.cols) * kBK + (kBM - g.rows) * kBK + (2 * kMaxStages + 2) * sizeof(uint64_t) + 16;
 }
 
 /* Tile t: groups of kGroupM row panels sweep the column panels together, so that the CTAs running at one
@@ -205,8 +211,9 @@ __device__ __forceinline__ void oz_tile(int t, int ntm, int ntn, int& bm, int& b
 __global__ void __launch_bounds__(kGemmThreads, 1) xs_ozaki_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* const smem = (unsigned char*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
-  const int ns = args.ns, nst = args.nstages;
-  const uint32_t abytes = (uint32_t)(ns * kSliceA), bbytes = (uint32_t)(ns * kSliceB), stage_bytes = abytes + bbytes;
+  const int ns = args.ns, nst = args.nstages, kps = args.kps;
+  const uint32_t abytes = (uint32_t)(ns * args.rows * kBK), bbytes = (uint32_t)(ns * args.cols * kBK); /* of a k block */
+  const uint32_t stage_bytes = (uint32_t)kps * (abytes + bbytes), stage_b = (uint32_t)kps * abytes;
   uint64_t* const bars = (uint64_t*)(smem + (size_t)nst * stage_bytes);
   uint64_t* const full = bars;
   uint64_t* const empty = bars + kMaxStages;
@@ -244,12 +251,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xs_ozaki_gemm_kernel(const __
         oz_tile(t, ntm, ntn, bm, bn);
         const unsigned char* const pa = args.dA + (size_t)bm * args.KB * abytes;
         const unsigned char* const pb = args.dB + (size_t)bn * args.KB * bbytes;
-        for (int kb = args.kb0; kb < args.kb1; ++kb) {
+        for (int kb = args.kb0; kb < args.kb1; kb += kps) {
+          const uint32_t nkb = (uint32_t)min(kps, args.kb1 - kb);
           if (!(ok = mbar_wait(&empty[stage], ph ^ 1u, abort, 1u, args.wait_limit))) break;
           unsigned char* const st = smem + (size_t)stage * stage_bytes;
-          mbar_arrive_expect_tx(&full[stage], stage_bytes);
-          bulk_load(st, pa + (size_t)kb * abytes, abytes, &full[stage]);
-          bulk_load(st + abytes, pb + (size_t)kb * bbytes, bbytes, &full[stage]);
+          mbar_arrive_expect_tx(&full[stage], nkb * (abytes + bbytes));
+          bulk_load(st, pa + (size_t)kb * abytes, nkb * abytes, &full[stage]);
+          bulk_load(st + stage_b, pb + (size_t)kb * bbytes, nkb * bbytes, &full[stage]);
           if (++stage == nst) {
             stage = 0;
             ph ^= 1u;
@@ -263,18 +271,34 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xs_ozaki_gemm_kernel(const __
       int stage = 0;
       uint32_t ph = 0u, use = 0u;
       bool ok = true;
+      OzOp few[kRegOps]; /* the MMAs of a k block, when they are that few, stay in registers */
+#pragma unroll
+      for (int i = 0; i < kRegOps; ++i) few[i] = args.op[1][i];
+      const int nfew = (kRegOps >= args.nops[1]) ? args.nops[1] : 0;
       for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++use) {
         if (!(ok = mbar_wait(acce, (use & 1u) ^ 1u, abort, 2u, args.wait_limit))) break;
         tc_fence_after();
-        for (int kb = args.kb0; kb < args.kb1; ++kb) {
+        for (int kb = args.kb0; kb < args.kb1; kb += kps) {
+          const int nkb = min(kps, args.kb1 - kb);
           if (!(ok = mbar_wait(&full[stage], ph, abort, 2u, args.wait_limit))) break;
           tc_fence_after();
-          const uint32_t a0 = smem_u32(smem + (size_t)stage * stage_bytes), b0 = a0 + abytes;
-          const int which = (kb == args.kb0) ? 0 : 1, n = args.nops[which];
-          for (int i = 0; i < n; ++i) {
-            const OzOp& o = args.op[which][i];
-            mma_i8(tmem + (uint32_t)(o.col * kBN), desc_k_noswz(a0 + o.sa * kSliceA, 128, 256),
-              desc_k_noswz(b0 + o.sb * kSliceB, 128, 256), idesc_i8(kBM, o.w * kBN), o.acc);
+          const uint32_t s0 = smem_u32(smem + (size_t)stage * stage_bytes);
+          uint64_t da = desc_k_noswz(s0, 128, 256), db = desc_k_noswz(s0 + stage_b, 128, 256);
+          for (int j = 0; j < nkb; ++j, da += abytes >> 4, db += bbytes >> 4) {
+            if (kb + j != args.kb0 && 0 != nfew) {
+#pragma unroll
+              for (int i = 0; i < kRegOps; ++i) {
+                if (i < nfew) mma_i8(tmem + (few[i].d & 0x7FFFFFFFu), da + few[i].a, db + few[i].b, few[i].idesc, 1u);
+              }
+              continue;
+            }
+            const int which = (kb + j == args.kb0) ? 0 : 1, n = args.nops[which];
+            const OzOp* const op = args.op[which];
+#pragma unroll 2
+            for (int i = 0; i < n; ++i) {
+              const OzOp o = op[i];
+              mma_i8(tmem + (o.d & 0x7FFFFFFFu), da + o.a, db + o.b, o.idesc, o.d >> 31);
+            }
           }
           mma_commit(&empty[stage]);
           if (++stage == nst) {
@@ -305,7 +329,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xs_ozaki_gemm_kernel(const __
       double w = w_last;
       for (int d = args.ndiag - 1; d >= 0; --d, w *= 128.0) {
         uint32_t v[32];
-        tmem_ld32(tbase + (uint32_t)(d * kBN), v);
+        tmem_ld32(tbase + (uint32_t)(d * args.cols), v);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 32; ++j) { /* exact int32 -> double: 2^52 + 2^31 + v, minus the offset */
@@ -369,9 +393,10 @@ int slice_operand(const double* x, long long ld, bool rows_contiguous, int R, in
 }
 
 /* The MMAs of a k block for the diagonals [d0, d0 + nd): per A slice its run of B slices, in pieces of at
-   most four slices (256 columns) of nearly equal width. first: a diagonal's first MMA writes its columns
+   most 256 columns of nearly equal width. first: a diagonal's first MMA writes its columns
    (a piece never mixes written and added columns). */
-int make_ops(int ns, int d0, int nd, bool first, OzOp* op) {
+int make_ops(int ns, int rows, int cols, int d0, int nd, bool first, OzOp* op) {
+  const int wmax = 256 / cols; /* slices per MMA */
   int n = 0, fresh = d0; /* diagonals from here on have not been written */
   for (int sa = 0; sa < ns; ++sa) {
     const int lo = max(0, d0 - sa), hi = min(ns - 1, d0 + nd - 1 - sa); /* B slices */
@@ -379,12 +404,11 @@ int make_ops(int ns, int d0, int nd, bool first, OzOp* op) {
       const bool acc = !first || sa + b < fresh;
       int e = hi; /* last slice of the run with the same accumulate flag */
       if (first && acc && sa + e >= fresh) e = fresh - 1 - sa;
-      const int len = e - b + 1, parts = (len + 3) / 4, w = (len + parts - 1) / parts;
-      op[n].sa = (unsigned char)sa;
-      op[n].sb = (unsigned char)b;
-      op[n].w = (unsigned char)w;
-      op[n].col = (unsigned char)(sa + b - d0);
-      op[n].acc = acc ? 1 : 0;
+      const int len = e - b + 1, parts = (len + wmax - 1) / wmax, w = (len + parts - 1) / parts;
+      op[n].a = (uint32_t)(sa * rows * kBK) >> 4;
+      op[n].b = (uint32_t)(b * cols * kBK) >> 4;
+      op[n].d = (uint32_t)((sa + b - d0) * cols) | (acc ? 1u << 31 : 0u);
+      op[n].idesc = idesc_i8(kBM, w * cols);
       ++n;
       b += w;
     }
@@ -393,14 +417,19 @@ int make_ops(int ns, int d0, int nd, bool first, OzOp* op) {
   return n;
 }
 
+/* Rows of a panel of A and columns of one of B: fewer than a tile's when there are no more (a panel's rows are
+   read and kept for every k, which for a product of a few rows and a long k would be most of the call). */
+int panel_rows(int M) { return M < kBM ? (M + 7) / 8 * 8 : kBM; }
+int panel_cols(int N) { return N < kBN ? (N + 15) / 16 * 16 : kBN; }
+
 }  // namespace
 
 extern "C" {
 
 size_t xs_ozaki_gemm_scratch_bytes(int M, int N, int K, int nslices) {
   const size_t Kp = align_up((size_t)(K > 0 ? K : 1), kBK);
-  return align_up((size_t)nslices * align_up(M, kBM) * Kp, 1024) + align_up((size_t)nslices * align_up(N, kBN) * Kp, 1024) +
-         align_up(sizeof(int) * M, 256) + align_up(sizeof(int) * N, 256) + 256;
+  return align_up((size_t)nslices * align_up(M, panel_rows(M)) * Kp, 1024) +
+         align_up((size_t)nslices * align_up(N, panel_cols(N)) * Kp, 1024) + align_up(sizeof(int) * M, 256) + align_up(sizeof(int) * N, 256) + 256;
 }
 
 int xs_ozaki_gemm(char transa, char transb, int M, int N, int K, double alpha, const double* a, int lda, const double* b,
@@ -420,12 +449,12 @@ int xs_ozaki_gemm(char transa, char transb, int M, int N, int K, double alpha, c
   if (nullptr == scratch || scratch_bytes < xs_ozaki_gemm_scratch_bytes(M, N, K, nslices)) return (int)cudaErrorInvalidValue;
   const int maxcut = 2 * (nslices - 1);
   if (cutoff < 0 || cutoff > maxcut) cutoff = maxcut;
-  const int Kp = (int)align_up((size_t)K, kBK);
+  const int Kp = (int)align_up((size_t)K, kBK), rows = panel_rows(M), cols = panel_cols(N);
   char* p = (char*)scratch;
   signed char* const dA = (signed char*)p;
-  p += align_up((size_t)nslices * align_up(M, kBM) * Kp, 1024);
+  p += align_up((size_t)nslices * align_up(M, rows) * Kp, 1024);
   signed char* const dB = (signed char*)p;
-  p += align_up((size_t)nslices * align_up(N, kBN) * Kp, 1024);
+  p += align_up((size_t)nslices * align_up(N, cols) * Kp, 1024);
   int* const ea = (int*)p;
   p += align_up(sizeof(int) * M, 256);
   int* const eb = (int*)p;
@@ -436,8 +465,8 @@ int xs_ozaki_gemm(char transa, char transb, int M, int N, int K, double alpha, c
   /* rows of op(A): A(i, k) at a[i + k*lda] ('N') or a[k + i*lda] ('T'); columns of op(B): B(k, j)
      at b[k + j*ldb] ('N', k contiguous) or b[j + k*ldb] ('T') */
   void* prof = xs_profile_begin(stream);
-  if (0 != (r = slice_operand(a, lda, !ta, M, K, Kp, nslices, kBM, ea, dA, s))) return r;
-  if (0 != (r = slice_operand(b, ldb, tb, N, K, Kp, nslices, kBN, eb, dB, s))) return r;
+  if (0 != (r = slice_operand(a, lda, !ta, M, K, Kp, nslices, rows, ea, dA, s))) return r;
+  if (0 != (r = slice_operand(b, ldb, tb, N, K, Kp, nslices, cols, eb, dB, s))) return r;
   xs_profile_end(prof, "ozaki_slice", 0.0, 8.0 * ((double)M * K + (double)K * N), stream);
   OzGemmArgs args;
   memset(&args, 0, sizeof(args));
@@ -457,10 +486,13 @@ int xs_ozaki_gemm(char transa, char transb, int M, int N, int K, double alpha, c
   args.dB = (const unsigned char*)dB;
   args.ns = nslices;
   args.KB = Kp / kBK;
+  args.rows = rows;
+  args.cols = cols;
+  args.kps = max(1, kStageBytes / (nslices * (rows + cols) * kBK));
   args.nstages = kMaxStages;
-  while (oz_gemm_smem(nslices, args.nstages) > 227 * 1024) --args.nstages;
+  while (oz_gemm_smem(args) > 227 * 1024) --args.nstages;
   /* at least 120 KB, so that an SM takes one CTA: it owns all tensor-memory columns */
-  const size_t smem = max((size_t)120 * 1024, oz_gemm_smem(nslices, args.nstages));
+  const size_t smem = max((size_t)120 * 1024, oz_gemm_smem(args));
   if (0 != (r = xs_func_smem((const void*)xs_ozaki_gemm_kernel, smem))) return r;
   const int ntiles = ((N + kBN - 1) / kBN) * ((M + kBM - 1) / kBM);
   for (int kb0 = 0; kb0 < args.KB; kb0 += kKChunkBlocks) {
@@ -470,8 +502,8 @@ int xs_ozaki_gemm(char transa, char transb, int M, int N, int K, double alpha, c
       args.ndiag = min(kMaxDiag, cutoff + 1 - d0);
       args.eshift = -2058 - 7 * d0;
       args.first = (0 == kb0 && 0 == d0) ? 1 : 0;
-      args.nops[0] = make_ops(nslices, d0, args.ndiag, true, args.op[0]);
-      args.nops[1] = make_ops(nslices, d0, args.ndiag, false, args.op[1]);
+      args.nops[0] = make_ops(nslices, rows, cols, d0, args.ndiag, true, args.op[0]);
+      args.nops[1] = make_ops(nslices, rows, cols, d0, args.ndiag, false, args.op[1]);
       prof = xs_profile_begin(stream);
       xs_ozaki_gemm_kernel<<<min(ntiles, xs_sm_count()), kGemmThreads, smem, s>>>(args);
       if (0 != (r = (int)cudaGetLastError())) return r;

@@ -38,6 +38,13 @@ def test_gemm_edges(acc, M, N, K, trans, slices, trim):
     assert np.max(np.abs(got - ref) / scale) <= TOL
 
 
+@pytest.mark.parametrize("M,N,K", [(8, 16, 64), (9, 17, 1300), (3, 40, 2000), (100, 5, 700), (130, 48, 40), (121, 49, 1000), (128, 1, 17000)])
+@pytest.mark.parametrize("slices,trim", [(1, 0), (2, 0), (3, 2), (4, 3), (8, 0)])
+def test_gemm_small_panels(acc, M, N, K, slices, trim):
+    """Panels of fewer rows or columns than a tile, several k blocks per stage and a last stage that is not full."""
+    test_gemm_edges(acc, M, N, K, "NT", slices, trim)
+
+
 @pytest.mark.parametrize("m,n,k", [(16, 16, 16), (33, 20, 40)])
 def test_stack_segment_over_many_chunks(acc, m, n, k):
     """One C block takes every entry, and a few blocks take many chunks each."""
