@@ -423,31 +423,33 @@ __device__ __forceinline__ double crt_value(const uint32_t (&S)[4], const Oz2Con
 }
 
 /* C(i,j) = alpha * x * 2^E + beta * C(i,j), x the centred integer with residues R[.][j][i]. A thread
-   takes four consecutive rows i (one 4-byte load per plane; planes have Mp rows, a multiple of 16), grid
-   rows take columns j (strided when N exceeds the grid).
+   takes V consecutive rows i (one V-byte load per plane; planes have Mp rows, a multiple of 16), grid
+   rows take columns j (strided when N exceeds the grid). Four rows need the fewest loads; one row per thread is faster
+   where that leaves the device a few waves (up to 303104 outputs; 201 x 203 outputs, 8 moduli, whole call: 42.2 -> 40.1 us).
    x / P = frac(sum_i r_i w_i) is summed as a 128-bit binary fraction: the wrap-around modulo 2^128
    takes the fractional part and the two's-complement reading of the sum centres it to [-1/2, 1/2)
    (x in [-P/2, P/2)). With w_i rounded down to 2^-128 the fraction is off by less than
    nmod * 255 * 2^-128 < 2^-115, i.e. x by less than 2^-115 P. The word columns are summed with wide integer
    multiply-adds: the same sums as exact doubles on the FP64 pipe took twice the time (4096 x 4096 outputs,
    16 moduli: 437 us against 223). */
-constexpr int kRecV = 4;
-__global__ void __launch_bounds__(256) xs_oz2_reconstruct(const unsigned char* __restrict__ R, int M, int N, int Mp,
+template <int V>
+__global__ void __launch_bounds__(256) xs_oz2_reconstruct(const unsigned char* __restrict__ R, int M, int N,
   const int* __restrict__ ea, const int* __restrict__ eb, const __grid_constant__ Oz2Consts cs, double alpha, double beta,
-  double* __restrict__ C, long long ldc) {
-  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * kRecV;
+  double* __restrict__ C, long long ldc, int Mp) {
+  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (i0 >= M) return;
   const size_t plane = (size_t)Mp * N;
-  int ia[kRecV];
+  int ia[V];
 #pragma unroll
-  for (int v = 0; v < kRecV; ++v) ia[v] = (i0 + v < M) ? ea[i0 + v] : 0;
-  /* four residues per word; the next column's loads are in flight while this column is computed */
+  for (int v = 0; v < V; ++v) ia[v] = (i0 + v < M) ? ea[i0 + v] : 0;
+  /* V residues per word; the next column's loads are in flight while this column is computed */
   unsigned res[kMaxMod], nxt[kMaxMod];
   auto load = [&](unsigned (&dst)[kMaxMod], int j) {
     const size_t off = (size_t)j * Mp + i0;
 #pragma unroll
     for (int q = 0; q < kMaxMod; ++q) {
-      dst[q] = (q < cs.nmod) ? *reinterpret_cast<const unsigned*>(R + (size_t)q * plane + off) : 0u;
+      if (4 == V) dst[q] = (q < cs.nmod) ? *reinterpret_cast<const unsigned*>(R + (size_t)q * plane + off) : 0u;
+      else dst[q] = (q < cs.nmod) ? R[(size_t)q * plane + off] : 0u;
     }
   };
   if (blockIdx.y < N) load(res, blockIdx.y);
@@ -456,7 +458,7 @@ __global__ void __launch_bounds__(256) xs_oz2_reconstruct(const unsigned char* _
     const int ib = eb[j];
     double* const cp = C + i0 + (long long)j * ldc;
 #pragma unroll
-    for (int v = 0; v < kRecV; ++v) {
+    for (int v = 0; v < V; ++v) {
       /* sum_i r_i w_i column by column: word k of the product sums to < 20 * 2^8 * 2^32 < 2^45 in
          64 bits, so no carry moves until the columns are combined (modulo 2^128) at the end */
       unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
@@ -469,12 +471,14 @@ __global__ void __launch_bounds__(256) xs_oz2_reconstruct(const unsigned char* _
         }
       }
       uint32_t S[4];
-      unsigned long long t = 0ull;
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        t = acc[w] + (t >> 32);
-        S[w] = (uint32_t)t;
-      }
+      unsigned long long t = acc[0];
+      S[0] = (uint32_t)t;
+      t = acc[1] + (t >> 32);
+      S[1] = (uint32_t)t;
+      t = acc[2] + (t >> 32);
+      S[2] = (uint32_t)t;
+      t = acc[3] + (t >> 32);
+      S[3] = (uint32_t)t;
       if (i0 + v < M) {
         const double val = (0 != ia[v] && 0 != ib) ? crt_value(S, cs, ia[v] + ib - 2150 + 2 * (53 - cs.mb)) : 0.0;
         cp[v] = (0.0 == beta) ? alpha * val : fma(alpha, val, beta * cp[v]);
@@ -545,6 +549,24 @@ double log2_product(int n) {
   return s;
 }
 
+/* The residue constants of every modulus, made by the compiler: a call of a small product would feel the divisions. */
+struct ModTables {
+  unsigned clo[kMaxMod] = {}, chi[kMaxMod] = {}, magic[kMaxMod] = {};
+  unsigned magic39[kMaxMod] = {}; /* floor(2^39 / m_i) + 1 */
+  constexpr ModTables() {
+    for (int i = 0; i < kMaxMod; ++i) {
+      const unsigned m = kModuli[i];
+      magic[i] = (unsigned)((1ull << 32) / m + 1ull);
+      magic39[i] = (unsigned)((1ull << 39) / m + 1ull);
+      for (int b = 0; b < 4; ++b) {
+        clo[i] |= (unsigned)((1ull << (8 * b)) % m) << (8 * b);
+        chi[i] |= (unsigned)((3 == b) ? (m - (1ull << 54) % m) % m : (1ull << (32 + 8 * b)) % m) << (8 * b);
+      }
+    }
+  }
+};
+constexpr ModTables kTables;
+
 /* Constants of the CRT with the first nmod moduli for inner dimension K. Returns the mantissa bits
    the inputs keep (0 if nmod cannot hold even one bit). */
 int make_consts(int nmod, int K, Oz2Consts* cs) {
@@ -573,13 +595,10 @@ int make_consts(int nmod, int K, Oz2Consts* cs) {
     cs->plo = (double)(Pld - (long double)cs->phi);
   }
   for (int i = 0; i < nmod; ++i) {
-    const unsigned m = kModuli[i];
-    cs->mod[i] = m;
-    cs->magic[i] = (unsigned)((1ull << 32) / m + 1ull);
-    for (int b = 0; b < 4; ++b) {
-      cs->clo[i] |= (unsigned)((1ull << (8 * b)) % m) << (8 * b);
-      cs->chi[i] |= (unsigned)((3 == b) ? (m - (1ull << 54) % m) % m : (1ull << (32 + 8 * b)) % m) << (8 * b);
-    }
+    cs->mod[i] = kModuli[i];
+    cs->magic[i] = kTables.magic[i];
+    cs->clo[i] = kTables.clo[i];
+    cs->chi[i] = kTables.chi[i];
   }
   for (int i = 0; i < nmod; ++i) {
     const unsigned m = kModuli[i];
@@ -694,7 +713,7 @@ int xs_ozaki2_gemm(char transa, char transb, int M, int N, int K, double alpha, 
   args.nmod = nmod;
   for (int i = 0; i < nmod; ++i) {
     args.mod[i] = cs.mod[i];
-    args.magic[i] = (unsigned)((1ull << 39) / cs.mod[i] + 1ull);
+    args.magic[i] = kTables.magic39[i];
   }
   args.R = rC;
   args.abort = abort;
@@ -719,8 +738,11 @@ int xs_ozaki2_gemm(char transa, char transb, int M, int N, int K, double alpha, 
   prof = xs_profile_begin(stream);
   const long long n = (long long)M * N;
   /* about four waves of resident blocks; each thread walks its columns */
-  const int rgx = (M + 256 * kRecV - 1) / (256 * kRecV), rgy = max(1, min(N, min(65535, 12 * xs_sm_count() / rgx)));
-  xs_oz2_reconstruct<<<dim3((unsigned)rgx, (unsigned)rgy), 256, 0, s>>>(rC, M, N, Mp, ea, eb, cs, alpha, beta, c, ldc);
+  const int V = (n <= 2048ll * xs_sm_count()) ? 1 : 4;
+  const int rgx = (M + 256 * V - 1) / (256 * V), rgy = max(1, min(N, min(65535, 12 * xs_sm_count() / rgx)));
+  const dim3 rgrid((unsigned)rgx, (unsigned)rgy);
+  if (4 == V) xs_oz2_reconstruct<4><<<rgrid, 256, 0, s>>>(rC, M, N, ea, eb, cs, alpha, beta, c, ldc, Mp);
+  else xs_oz2_reconstruct<1><<<rgrid, 256, 0, s>>>(rC, M, N, ea, eb, cs, alpha, beta, c, ldc, Mp);
   r = (int)cudaGetLastError();
   xs_profile_end(prof, "ozaki2_reconstruct", 0.0, (double)nmod * n + 16.0 * n, stream);
   return r;
