@@ -73,8 +73,14 @@ typedef struct xs_smm_params_t {
   int generic; /* 1: always use the runtime-shape kernel even if a specialised one exists */
   int wpb;     /* warps per CTA */
   int sorted;  /* 1: the stack is known to be grouped by c (skip the device sort) */
-  int tile;    /* 1: not a tuned record, so the tile kernel may take the stack where it is the faster one */
+  int tile;    /* 1: the tile kernel may take the stack where it is the faster one (not for records that a file or
+                  libxstream_b200_set_params gave) */
 } xs_smm_params_t;
+
+/** Which kernel runs a stack: on the tile kernel mt, nt, kp and wpb have no meaning. */
+enum { XS_KERNEL_REGISTER = 0, XS_KERNEL_STAGED = 1, XS_KERNEL_FMA = 2, XS_KERNEL_TILE = 3 };
+/** The kernel of a stack (of its first part, when it is processed in parts); -1 if there is none. */
+int xs_smm_kernel_kind(int stack_size, int m, int n, int k, const xs_smm_params_t* params);
 
 /** kp value that selects the register-blocked FMA stack kernel (small blocks). */
 #define XS_KP_FMA (-1)

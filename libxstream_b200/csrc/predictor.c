@@ -106,6 +106,7 @@ void xs_autotune_if_needed(int m, int n, int k, int stack_size, void* stream) {
   if (!xs_autotune_enabled()) return;
   xs_params_lookup_ex(3, m, n, k, stack_size, &p, &source);
   if (XS_PARAMS_TUNED == source || XS_PARAMS_PREDICTED == source) return;
+  if (XS_KERNEL_TILE == xs_smm_kernel_kind(stack_size, m, n, k, &p)) return; /* runs on none of the candidates */
   if (cudaSuccess != cudaStreamIsCapturing((cudaStream_t)stream, &cs) || cudaStreamCaptureStatusNone != cs) return;
   nc = xs_tune_candidates(m, n, cand, 33);
   if (nc > 33) return;
@@ -124,6 +125,7 @@ void xs_autotune_if_needed(int m, int n, int k, int stack_size, void* stream) {
     p.wpb = 4;
     p.generic = 0;
     p.sorted = 0;
+    p.tile = 1; /* the record is for the stacks that the tile kernel does not take */
     xs_params_set(3, m, n, k, &p, 2e-6 * m * n * k * (double)stack_size / ms[best]);
     if (2 <= xs_verbosity()) {
       fprintf(stderr, "INFO LIBSMM/B200: tuned %ix%ix%i S=%i: mt=%i nt=%i kp=%i (%.3f ms)\n", m, n, k, stack_size, p.mt, p.nt,

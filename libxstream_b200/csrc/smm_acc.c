@@ -162,8 +162,9 @@ static int xs_process_format(const int* dev_param_stack, int stack_size, int for
   xs_autotune_if_needed(m_max, n_max, k_max, stack_size, stream);
   xs_params_lookup((int)datatype, m_max, n_max, k_max, stack_size, &prm);
   if (3 <= xs_verbosity()) {
-    fprintf(stderr, "INFO LIBSMM/B200: SMM-kernel %ix%ix%i L=%i MT=%i NT=%i KP=%i WPB=%i ss=%i\n", m_max, n_max, k_max,
-      prm.chunk, prm.mt, prm.nt, prm.kp, prm.wpb, stack_size);
+    fprintf(stderr, "INFO LIBSMM/B200: SMM-kernel %ix%ix%i L=%i MT=%i NT=%i KP=%i WPB=%i ss=%i%s\n", m_max, n_max, k_max,
+      prm.chunk, prm.mt, prm.nt, prm.kp, prm.wpb, stack_size,
+      XS_KERNEL_TILE == xs_smm_kernel_kind(stack_size, m_max, n_max, k_max, &prm) ? " (tile kernel)" : "");
   }
   nbytes = xs_smm_f64_scratch_bytes(stack_size, m_max, n_max, k_max, &prm);
   result = xs_scratch_alloc(&scratch, nbytes, stream);
@@ -263,6 +264,7 @@ int libxstream_b200_set_params(int m, int n, int k, int chunk, int mt, int nt, i
   p.wpb = wpb;
   p.sorted = 0;
   p.generic = 0;
+  p.tile = 0; /* runs as it says */
   return xs_params_set((int)dbcsr_type_real_8, m, n, k, &p, 0.0);
 }
 

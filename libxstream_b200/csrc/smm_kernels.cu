@@ -1905,6 +1905,16 @@ cudaError_t launch_unsupported(const SmmPlan&, const StackTask&, int*, const uns
   return cudaErrorInvalidValue;
 }
 
+/* Whether a staged kernel of either kind runs the shape with these parameters. */
+bool staged_listed(int m, int n, int k, const xs_smm_params_t* prm) {
+  if ((m + 7) / 8 != prm->mt || (n + 7) / 8 != prm->nt) return false;
+  if (4 < prm->wpb && nullptr != find_ws(m, n, k, prm->wpb)) return true;
+  for (const SpecEntry& e : staged_table) {
+    if (e.m == m && e.n == n && e.k == k) return true;
+  }
+  return false;
+}
+
 launch_fn_t find_launcher(int m, int n, int k, const xs_smm_params_t* prm) {
   if (XS_KP_FMA == prm->kp) {
     const FmaEntry* const f = find_fma(m, n, k);
@@ -2282,6 +2292,15 @@ size_t xs_smm_f64_scratch_bytes(int stack_size, int m, int n, int k, const xs_sm
   if (stack_size > xs_stack_group_max()) stack_size = xs_stack_group_max(); /* processed in parts */
   if (0 >= stack_size || 0 != plan_smm(stack_size, m, n, k, params, &pl)) return 0;
   return pl.total;
+}
+
+int xs_smm_kernel_kind(int stack_size, int m, int n, int k, const xs_smm_params_t* params) {
+  SmmPlan pl;
+  if (stack_size > xs_stack_group_max()) stack_size = xs_stack_group_max();
+  if (0 >= stack_size || 0 != plan_smm(stack_size, m, n, k, params, &pl)) return -1;
+  if (pl.tile) return XS_KERNEL_TILE;
+  if (XS_KP_FMA == params->kp) return XS_KERNEL_FMA;
+  return (0 == params->generic && staged_listed(m, n, k, params)) ? XS_KERNEL_STAGED : XS_KERNEL_REGISTER;
 }
 
 int xs_launch_smm_f64(const int* dev_stack, int S, const double* a, const double* b, double* c, int m, int n, int k,

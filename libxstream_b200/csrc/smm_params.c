@@ -42,6 +42,7 @@ static void xs_sanitize(xs_smm_params_t* p) {
   p->generic = (0 != p->generic) ? 1 : 0;
   p->wpb = xs_clamp(p->wpb, 1, 16); /* above 4: consumer warps of a warp-specialised kernel */
   p->sorted = (0 != p->sorted) ? 1 : 0;
+  p->tile = (0 != p->tile) ? 1 : 0;
 }
 
 /* Tiles of at most 4x4 DMMA fragments per warp; prefer the split of ceil(x/8) fragments into
@@ -162,7 +163,6 @@ int xs_params_set(int type, int m, int n, int k, const xs_smm_params_t* p, doubl
         r->k = k;
         r->gflops = gflops;
         r->p = *p;
-        r->p.tile = 0; /* tuned records run as they say */
         xs_sanitize(&r->p);
       }
       result = 0;
@@ -206,6 +206,7 @@ int xs_params_load_csv(const char* path) {
       p.wpb = atoi(fields[11]);
       p.sorted = 0;
       p.generic = (13 <= nf) ? atoi(fields[12]) : 0;
+      p.tile = 0; /* a record of a file runs as it says */
       if (0 < m && 0 < n && 0 < k && 0 == xs_params_set(type, m, n, k, &p, gflops)) ++count;
     }
   }
