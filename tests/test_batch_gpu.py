@@ -12,6 +12,7 @@ import pytest
 import oracle
 from libxstream_b200 import StackDesc
 from libxstream_b200 import workloads as W
+from test_kernel_choice import FMA, STAGED, TILE, kind, record
 
 pytestmark = pytest.mark.gpu
 
@@ -164,10 +165,10 @@ def test_batch_rejects_unsuitable_stacks(acc):
 
 
 def test_batch_mixed_item_kinds(acc):
-    """Large and small stacks of the same shapes in one persistent launch: 23^3 and 16x64x9 items run
-    their staged item functions (16x64x9 with a 2 x 8-fragment tile), 45^3 items the register kernel
-    with sub-tiles; every stack combines its CTA-crossing segments in the kernel. Parity and bitwise
-    reproducibility."""
+    """Large and small stacks of the same shapes: the two large ones run their staged kernels in launches of
+    their own, 23^3 and 16x64x9 items of the small ones their staged item functions (16x64x9 with a 2 x 8-fragment tile),
+    45^3 items the register kernel with sub-tiles; every stack combines its CTA-crossing segments in the kernel.
+    Parity and bitwise reproducibility."""
     A, stream = acc
     cases = [W.stack_case(16, 64, 9, 120000, 2000, 2000, 500, seed=701),
              W.stack_case(16, 64, 9, 900, 100, 100, 30, seed=702),
@@ -185,3 +186,63 @@ def test_batch_mixed_item_kinds(acc):
     for d, got in zip(devs, first):
         assert np.array_equal(d.result(stream), got)
         d.free()
+
+
+def check_batch(A, stream, cases, launches):
+    """Parity, the same bits from call to call, and a captured call of `launches` kernels that adds the stacks again."""
+    lib = A.lib()
+    devs = [DevCase(A, stream, c, c0=W.rng(i).uniform(-1, 1, size=c.nc * c.m * c.n)) for i, c in enumerate(cases)]
+    assert run_batch(A, stream, devs) == 0
+    first = [d.result(stream) for d in devs]
+    for d, got in zip(devs, first):
+        assert oracle.block_relerr(got, d.reference(), d.case.m * d.case.n) <= TOL, (d.case.m, d.case.n, d.case.k)
+        d.c.upload(d.c0, stream)
+    assert run_batch(A, stream, devs) == 0
+    for d, got in zip(devs, first):
+        assert np.array_equal(d.result(stream), got)
+    gexec, nk = ctypes.c_void_p(), ctypes.c_int(0)
+    assert lib.libxstream_b200_graph_begin(stream.handle) == 0
+    rc = run_batch(A, stream, devs)
+    assert lib.libxstream_b200_graph_end(stream.handle, ctypes.byref(gexec), ctypes.byref(nk)) == 0
+    assert rc == 0 and nk.value == launches
+    assert lib.libxstream_b200_graph_launch(gexec, stream.handle) == 0
+    stream.sync()
+    assert lib.libxstream_b200_graph_destroy(gexec) == 0
+    for d in devs:
+        assert oracle.block_relerr(d.result(stream), d.reference(times=2), d.case.m * d.case.n) <= TOL
+        d.free()
+
+
+def test_batch_parts_launched_alone_beside_the_persistent_kernel(acc):
+    """A part on the tile kernel, one on the FMA kernel (which sizes its pieces differently), one of many tiny entries, one
+    staged part, each in a launch of its own, and small parts in the persistent kernel."""
+    A, stream = acc
+    try:
+        record(6, 6, 18, 1, 1, -1, 1)  # kp = -1: the FMA kernel
+        assert kind(45, 26, 22, 20000) == TILE and kind(6, 6, 18, 40000) == FMA and kind(23, 23, 23, 90000) == STAGED
+        cases = [W.stack_case(45, 26, 22, 20000, 500, 500, 300, seed=801, zipf_s=1.1),
+                 W.stack_case(6, 6, 18, 40000, 2000, 2000, 900, seed=802, zipf_s=1.1),
+                 W.stack_case(32, 5, 5, 40000, 2000, 2000, 900, seed=803),
+                 W.stack_case(23, 23, 23, 90000, 2000, 2000, 400, seed=804),
+                 W.stack_case(13, 13, 13, 900, 90, 90, 30, seed=805),
+                 W.stack_case(45, 45, 45, 500, 50, 50, 20, seed=806),
+                 W.stack_case(9, 4, 5, 777, 70, 70, 25, seed=807)]
+        check_batch(A, stream, cases, 6)  # the grouping, four parts alone, the persistent kernel
+    finally:
+        A.lib().libxstream_b200_clear_params()
+
+
+def test_batch_of_large_parts_only(acc):
+    """Nothing is left for the persistent kernel."""
+    A, stream = acc
+    cases = [W.stack_case(45, 45, 45, 5000, 200, 200, 100, seed=811), W.stack_case(64, 64, 64, 2000, 100, 100, 60, seed=812),
+             W.stack_case(7, 10, 5, 33000, 2000, 2000, 900, seed=813)]
+    check_batch(A, stream, cases, 4)
+
+
+def test_batch_large_staged_stacks_in_the_persistent_kernel(acc):
+    """Staged parts just below the size from which they are launched alone (4e6 DMMA steps)."""
+    A, stream = acc
+    cases = [W.stack_case(23, 23, 23, 70000, 2000, 2000, 400, seed=821, zipf_s=1.1), W.stack_case(16, 64, 9, 80000, 2000, 2000, 500, seed=822),
+             W.stack_case(23, 23, 23, 300, 50, 50, 20, seed=823)]
+    check_batch(A, stream, cases, 2)

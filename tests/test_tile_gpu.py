@@ -13,6 +13,7 @@ import pytest
 
 import oracle
 from libxstream_b200 import workloads as W
+from test_kernel_choice import TILE, kind
 
 pytestmark = pytest.mark.gpu
 
@@ -71,6 +72,22 @@ def test_shapes(acc, shape, shift):
     case = W.stack_case(m, n, k, S, 60, 50, 90, seed=m + 100 * n + 10000 * k)
     got = run(A, stream, case, shift)
     assert oracle.block_relerr(got, reference(case), m * n) <= TOL
+
+
+# one DMMA step per panel, tiles of 4 x 4 on two padded operands, a team of two 4 x 4 tiles over several panels
+@pytest.mark.parametrize("m,n,k,S", [(69, 28, 3, 20100), (64, 64, 64, 1600), (54, 29, 73, 1400), (23, 22, 5, 40100)])
+def test_more_shapes(acc, m, n, k, S):
+    A, stream = acc
+    assert kind(m, n, k, S) == TILE
+    case = W.stack_case(m, n, k, S, 60, 50, 90, seed=S)
+    assert oracle.block_relerr(run(A, stream, case, 1), reference(case), m * n) <= TOL
+
+
+def test_the_tile_kernel_runs_them(acc):
+    """The stacks of this file, but for two shapes of test_shapes that run faster on the register kernel at that size."""
+    others = {s for s in SHAPES if kind(*s, int(7.2e5 / steps(*s)) + 3) != TILE}
+    assert others == {(64, 64, 64), (80, 73, 3)}
+    assert kind(45, 45, 45, 3000) == kind(40, 33, 24, 8000) == TILE
 
 
 @pytest.mark.parametrize("nc,zipf", [(1, 0.0), (3, 1.1), (2900, 0.0)])
