@@ -1614,12 +1614,12 @@ static bool use_tile(int m, int n, int k, int S, const xs_smm_params_t* prm) {
 
 static bool spec_listed(int m, int n, int k, const xs_smm_params_t* prm);
 
-/* The tile kernel's plan of a stack, if it takes it. Teams of 4 x 4 tiles are eight warps per SM, which need five
+/* The tile kernel's plan of a stack, if it takes it. Teams of 4 x 4 tiles are eight warps per SM, which need four
    entries each to win over a register kernel compiled for the very shape (64^3 in uniform C blocks: 832 entries
-   40 us against 45, 1173: 48 against 54, 1465: 57 against 59; 1500: 63 against 62; 2930: 98 against 94). */
+   40 us against 45, 1173: 48 against 54, 1465: 57 against 59, 2930: 98 against 94; in Zipf ones 1173: 50 against 48). */
 static bool plan_tile(int S, int m, int n, int k, const xs_smm_params_t* prm, xs_tile_plan_t* tp) {
   if (!use_tile(m, n, k, S, prm) || 0 != xs_tile_plan(S, m, n, k, tp)) return false;
-  return 12 >= tp->mt * tp->nt || !spec_listed(m, n, k, prm) || S >= 5l * tp->ctas * tp->nteam * xs_sm_count();
+  return 12 >= tp->mt * tp->nt || !spec_listed(m, n, k, prm) || S >= 4l * tp->ctas * tp->nteam * xs_sm_count();
 }
 
 int plan_smm(int S, int m, int n, int k, const xs_smm_params_t* prm, SmmPlan* pl) {
@@ -2016,9 +2016,9 @@ constexpr int kSoloEntries = 32768;
 /* Work decomposition of a batch for the unified kernel: stacks split into parts of at most
    xs_stack_group_max() entries; per part its kernel (the staged item function of its shape, or the
    register kernel of a tile class of at most 4 x 4 fragments) and a chunk length L chosen so that every
-   work item (kUniW chunks x one sub-tile) costs about the same (kUniItemsMin..kUniItemsMax items per
-   resident CTA). Returns the
-   number of parts, -1 if the batch has too many parts or the kernel cannot be set up. */
+   work item (kUniW chunks x one sub-tile) costs about the same (one item per
+   resident CTA for a single part, else kUniItemsMin, or kUniItemsMinRest beside parts launched alone, to
+   kUniItemsMax). Returns the number of parts, -1 if the batch has too many parts or the kernel cannot be set up. */
 int plan_uni(const libxstream_b200_stack_t* st, int ns, UniPlan* up) {
   const int smax = xs_stack_group_max();
   up->nparts = 0;

@@ -603,15 +603,23 @@ int xs_tile_geometry(int m, int n, int k, xs_tile_plan_t* pl) {
   pl->ctas = ctas;
   /* DMMA instructions of a warp in a panel: they have to pay for the panel's wait, the team's barrier and, where
      columns are padded, the copies that the team issues itself. Over 1230 stacks (all shapes up to 80, 7e5 to 5e6
-     steps) these lines leave out what was up to 1.4 times slower than the register kernel and, in the mean, as fast:
-     - panels of one or two DMMA steps (k <= 8) without padding only (32x76x5, 12502 entries: register kernel 65 us,
-       this one 83), with a second team beside them (77x64x7, 6252: 63, 79), and of at least 8 or 18 instructions
-       (7x72x7, 88890: 153, 178; 46x13x5, 192109: 228, 256; but 23x22x5, 88890: 99, 93);
-     - padded columns: never for a lone warp (16x32x64, 6252: 45, 52), and for a team of two in short entries only
-       from 25 instructions on (9x48x13, 33335: 86, 94; but 48x45x9, 46298: 251, 230). */
+     steps) these lines leave out what was up to 1.4 times slower than the register kernel, 5 % in the mean:
+     - panels of one or two DMMA steps (k <= 8) with padded columns and fewer than three teams on an SM (32x76x5, 12502
+       entries: register kernel 65 us, this one 83), in the only team of an SM, unless it is of ten warps (74x58x6,
+       10002: 86, 99; 77x76x4, 8002: 96, 74), and of fewer than 8 (one step) or 18 (two) instructions: 7x72x7, 88890: 153, 178;
+       46x13x5, 192109: 228, 256. With one row or column of fragments 8 are enough for two steps (4x78x8);
+     - padded columns and a lone warp, unless it copies 32-wide columns or wider ones of one operand for at least eight
+       fragments (16x32x64, 6252: 45, 52; 16x9x45, 17710: 47, 55; but 13x32x45, 52085: 0.93 of the time). */
   const int psteps = (min(pl->pk, k) - 1) / 4 + 1, instr = c.mt * c.nt * psteps;
-  if (2 >= psteps && (0 < padded || 1 == ctas * c.nteam || instr < (1 == psteps ? 8 : 18))) return -1;
-  if (0 < padded && (1 == c.T || (2 == c.T && 1 == pl->npan && instr < 25))) return -1;
+  if (2 >= psteps) {
+    if (0 < padded && 3 > ctas * c.nteam) return -1;
+    if (1 == ctas * c.nteam && 10 > c.T) return -1;
+    if (instr < (1 == psteps || 8 >= m || 8 >= n ? 8 : (10 > c.T ? 18 : 0))) return -1;
+  }
+  if (0 < padded && 1 == c.T) {
+    const int side = (0 == m % 16) ? m : n;
+    if (2 == padded || (10 > c.mt * c.nt && (8 > c.mt * c.nt || 16 == side))) return -1;
+  }
   pl->smem = (size_t)geo.region * c.nteam + slack;
   return 0;
 }

@@ -52,7 +52,7 @@ def test_kinds(acc):
     assert kind(45, 45, 45, 3000) == TILE and kind(45, 45, 45, 1000) == REGISTER  # 7e5 DMMA steps are 1621 entries
     assert kind(23, 23, 23, 3000) == kind(23, 23, 23, 300000) == STAGED
     assert kind(46, 13, 5, 100000) == REGISTER  # 12 DMMA instructions per warp and panel
-    assert kind(64, 64, 64, 1400) == REGISTER and kind(64, 64, 64, 1500) == TILE
+    assert kind(64, 64, 64, 1100) == REGISTER and kind(64, 64, 64, 1200) == TILE
     assert kind(45, 45, 45, 2000000) == TILE  # in parts
     try:
         record(45, 45, 45, 3, 3, 2, 1)

@@ -59,7 +59,7 @@ def test_blocks_beyond_ten_warps_are_refused():
 
 
 @pytest.mark.parametrize("m,n,k", [(46, 13, 5), (9, 39, 8), (7, 72, 7), (12, 70, 3), (32, 76, 5), (64, 64, 5), (77, 64, 7), (74, 58, 6),
-                                   (71, 78, 3), (16, 32, 64), (32, 4, 64), (16, 9, 45), (9, 48, 13), (22, 32, 16), (13, 16, 9)])
+                                   (71, 78, 3), (16, 32, 64), (32, 4, 64), (16, 9, 45), (64, 75, 6), (13, 16, 9)])
 def test_panels_with_too_little_work_are_refused(m, n, k):
     """Shapes measured slower than on the register kernel: few DMMA instructions per warp and panel, one team per SM,
     padded columns for one or two warps."""
@@ -67,7 +67,7 @@ def test_panels_with_too_little_work_are_refused(m, n, k):
 
 
 @pytest.mark.parametrize("m,n,k", [(45, 45, 45), (64, 64, 64), (17, 29, 11), (32, 32, 32), (45, 26, 22), (13, 22, 9), (23, 22, 5), (48, 45, 9),
-                                   (69, 28, 3), (80, 80, 80), (54, 29, 73), (72, 72, 16), (40, 33, 24), (9, 10, 20)])
+                                   (69, 28, 3), (80, 80, 80), (54, 29, 73), (72, 72, 16), (40, 33, 24), (9, 10, 20), (77, 76, 4), (13, 32, 35), (22, 32, 16), (4, 78, 8), (37, 16, 18)])
 def test_shapes_measured_faster_are_taken(m, n, k):
     pl = geometry(m, n, k)
     assert pl is not None and pl.T * pl.nteam * pl.ctas >= 8
