@@ -24,7 +24,7 @@
  * exponents ea[M], eb[N], residues of C R[q][N][Mp] (u8, column-major per modulus,
  * Mp = M rounded up to 16).
  *
- * GEMM kernel: persistent, one CTA per SM, 10 warps, the pipeline of the scheme-1 kernel over work
+ * GEMM kernel: persistent, one CTA per SM, 10 warps, a pipeline of copies, MMAs and epilogue over work
  * units (modulus, 128 x 256 tile of C) taken modulus-major and strided by the grid: warp 0 streams
  * the k-blocks of both operands' residue planes into a 4-stage shared-memory ring with TMA (128-byte
  * swizzle); warp 1 owns two 128 x 256 int32 accumulators in tensor memory and one lane issues the

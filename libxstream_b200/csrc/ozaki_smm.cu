@@ -8,7 +8,7 @@
  *    ozaki_common.cl:789-834 and the per-row/per-column exponents of ozaki1_int8.cl:428-589, applied
  *    to each block). Digits are stored MMA-ready: per block and slice a K-major tile of
  *    rows8 x KP bytes (rows rounded up to 8 for A, 16 for B; KP = k rounded up to 32) made of core
- *    matrices of 8 rows x 16 bytes; exponents per block row / column.
+ *    matrices of 8 rows x 16 bytes; a scale per block row / column.
  * 2. The stack is grouped by c (the plain path's grouping sort) and cut into chunks of L entries,
  *    one CTA per chunk (18 warps, 1 CTA per SM).
  * 3. Per entry, warp 0 copies the entry's A and B digit tiles into a shared-memory stage with bulk
@@ -49,7 +49,7 @@ constexpr int kTmemCols = 512;
 constexpr unsigned kErrOzakiTimeout = 4u;
 constexpr unsigned kErrBadOffset = 8u;
 constexpr int kMaxChunk = 1024; /* entries per chunk (their keys are staged in shared memory) */
-constexpr int kXSlots = 8;      /* exponent ring: row exponents of A and column exponents of B per entry */
+constexpr int kXSlots = 8;      /* scale ring: row scales of A and column scales of B per entry */
 
 /* ------------------------------------------------------------------------- pool slicing */
 
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1) xs_ozs_smm_kernel(const __grid_co
       }
     }
   }
-  else { /* epilogue: warps 2..9 */
+  else { /* epilogue: warps 2..17 */
     const int q = warp & 3, part = (warp - 2) >> 2;
     const int row = 16 * q + lane;
     const bool rok = (lane < 16) && (row < g.m);
@@ -469,7 +469,7 @@ int plan_oz(int m, int n, int k, int ns, int cutoff, OzPlan* p) {
 }
 
 struct OzLayout {
-  size_t dA, dB, eA, eB, keys0, keys1, keys2, vals0, vals1, vals2, pieces, sort, abort, total;
+  size_t dA, dB, wA, wB, keys0, keys1, keys2, vals0, vals1, vals2, pieces, sort, abort, total;
   int L, nchunks;
 };
 
@@ -485,9 +485,9 @@ void layout_oz(const OzPlan& p, int S, int m, int n, int na, int nb, OzLayout* l
   o = align_up(o + p.poolA * (size_t)na, 256);
   l->dB = o;
   o = align_up(o + p.poolB * (size_t)nb, 256);
-  l->eA = o;
+  l->wA = o;
   o = align_up(o + sizeof(double) * 64 * (size_t)na, 256);
-  l->eB = o;
+  l->wB = o;
   o = align_up(o + sizeof(double) * 64 * (size_t)nb, 256);
   const size_t ks = align_up(sizeof(unsigned) * (size_t)part, 256), vs = align_up(sizeof(unsigned long long) * (size_t)part, 256);
   l->keys0 = o;
@@ -535,8 +535,8 @@ int xs_launch_smm_ozaki(const int* dev_stack, int S, int m, int n, int k, const 
   char* const base = (char*)scratch;
   unsigned char* const dA = (unsigned char*)(base + l.dA);
   unsigned char* const dB = (unsigned char*)(base + l.dB);
-  double* const wA = (double*)(base + l.eA);
-  double* const wB = (double*)(base + l.eB);
+  double* const wA = (double*)(base + l.wA);
+  double* const wB = (double*)(base + l.wB);
   unsigned* const abort = (unsigned*)(base + l.abort);
   int r = (int)cudaMemsetAsync(abort, 0, 256, s);
   if (0 != r) return r;
