@@ -442,20 +442,24 @@ __global__ void __launch_bounds__(256) xs_oz2_reconstruct(const unsigned char* _
   int ia[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) ia[v] = (i0 + v < M) ? ea[i0 + v] : 0;
-  /* V residues per word; the next column's loads are in flight while this column is computed */
+  /* V residues per word; the next column's loads, its exponent's too, are in flight while this column is computed */
   unsigned res[kMaxMod], nxt[kMaxMod];
   auto load = [&](unsigned (&dst)[kMaxMod], int j) {
     const size_t off = (size_t)j * Mp + i0;
 #pragma unroll
     for (int q = 0; q < kMaxMod; ++q) {
-      if (4 == V) dst[q] = (q < cs.nmod) ? *reinterpret_cast<const unsigned*>(R + (size_t)q * plane + off) : 0u;
+      /* planes beyond the last modulus: the first one's residues, not used (a predicate on every word cost 12 registers and
+         10 % of the time) */
+      if (4 == V) dst[q] = *reinterpret_cast<const unsigned*>(R + (size_t)(q < cs.nmod ? q : 0) * plane + off);
       else dst[q] = (q < cs.nmod) ? R[(size_t)q * plane + off] : 0u;
     }
   };
+  int ibn = (blockIdx.y < N) ? eb[blockIdx.y] : 0;
   if (blockIdx.y < N) load(res, blockIdx.y);
   for (int j = blockIdx.y; j < N; j += gridDim.y) {
     if (j + gridDim.y < N) load(nxt, j + gridDim.y);
-    const int ib = eb[j];
+    const int ib = ibn;
+    if (j + gridDim.y < N) ibn = eb[j + gridDim.y];
     double* const cp = C + i0 + (long long)j * ldc;
 #pragma unroll
     for (int v = 0; v < V; ++v) {
@@ -739,10 +743,11 @@ int xs_ozaki2_gemm(char transa, char transb, int M, int N, int K, double alpha, 
   const long long n = (long long)M * N;
   /* about four waves of resident blocks; each thread walks its columns */
   const int V = (n <= 2048ll * xs_sm_count()) ? 1 : 4;
-  const int rgx = (M + 256 * V - 1) / (256 * V), rgy = max(1, min(N, min(65535, 12 * xs_sm_count() / rgx)));
+  const int bt = (M <= 64 * V) ? 64 : (M <= 128 * V) ? 128 : 256; /* threads that have rows */
+  const int rgx = (M + bt * V - 1) / (bt * V), rgy = max(1, min(N, min(65535, 12 * xs_sm_count() / rgx)));
   const dim3 rgrid((unsigned)rgx, (unsigned)rgy);
-  if (4 == V) xs_oz2_reconstruct<4><<<rgrid, 256, 0, s>>>(rC, M, N, ea, eb, cs, alpha, beta, c, ldc, Mp);
-  else xs_oz2_reconstruct<1><<<rgrid, 256, 0, s>>>(rC, M, N, ea, eb, cs, alpha, beta, c, ldc, Mp);
+  if (4 == V) xs_oz2_reconstruct<4><<<rgrid, bt, 0, s>>>(rC, M, N, ea, eb, cs, alpha, beta, c, ldc, Mp);
+  else xs_oz2_reconstruct<1><<<rgrid, bt, 0, s>>>(rC, M, N, ea, eb, cs, alpha, beta, c, ldc, Mp);
   r = (int)cudaGetLastError();
   xs_profile_end(prof, "ozaki2_reconstruct", 0.0, (double)nmod * n + 16.0 * n, stream);
   return r;

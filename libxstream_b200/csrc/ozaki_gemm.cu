@@ -208,6 +208,7 @@ __device__ __forceinline__ void oz_tile(int t, int ntm, int ntn, int& bm, int& b
   bn = r / gsize;
 }
 
+template <bool FEW>
 __global__ void __launch_bounds__(kGemmThreads, 1) xs_ozaki_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* const smem = (unsigned char*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xs_ozaki_gemm_kernel(const __
       OzOp few[kRegOps]; /* the MMAs of a k block, when they are that few, stay in registers */
 #pragma unroll
       for (int i = 0; i < kRegOps; ++i) few[i] = args.op[1][i];
-      const int nfew = (kRegOps >= args.nops[1]) ? args.nops[1] : 0;
+      const int nfew = args.nops[1];
       for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++use) {
         if (!(ok = mbar_wait(acce, (use & 1u) ^ 1u, abort, 2u, args.wait_limit))) break;
         tc_fence_after();
@@ -285,7 +286,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xs_ozaki_gemm_kernel(const __
           const uint32_t s0 = smem_u32(smem + (size_t)stage * stage_bytes);
           uint64_t da = desc_k_noswz(s0, 128, 256), db = desc_k_noswz(s0 + stage_b, 128, 256);
           for (int j = 0; j < nkb; ++j, da += abytes >> 4, db += bbytes >> 4) {
-            if (kb + j != args.kb0 && 0 != nfew) {
+            if (FEW && kb + j != args.kb0) {
 #pragma unroll
               for (int i = 0; i < kRegOps; ++i) {
                 if (i < nfew) mma_i8(tmem + (few[i].d & 0x7FFFFFFFu), da + few[i].a, db + few[i].b, few[i].idesc, 1u);
@@ -327,9 +328,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) xs_ozaki_gemm_kernel(const __
 #pragma unroll
       for (int j = 0; j < 32; ++j) sum[j] = 0.0;
       double w = w_last;
+      uint32_t at = tbase + (uint32_t)(args.ndiag * args.cols);
       for (int d = args.ndiag - 1; d >= 0; --d, w *= 128.0) {
         uint32_t v[32];
-        tmem_ld32(tbase + (uint32_t)(d * args.cols), v);
+        at -= (uint32_t)args.cols;
+        tmem_ld32(at, v);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 32; ++j) { /* exact int32 -> double: 2^52 + 2^31 + v, minus the offset */
@@ -493,7 +496,6 @@ int xs_ozaki_gemm(char transa, char transb, int M, int N, int K, double alpha, c
   while (oz_gemm_smem(args) > 227 * 1024) --args.nstages;
   /* at least 120 KB, so that an SM takes one CTA: it owns all tensor-memory columns */
   const size_t smem = max((size_t)120 * 1024, oz_gemm_smem(args));
-  if (0 != (r = xs_func_smem((const void*)xs_ozaki_gemm_kernel, smem))) return r;
   const int ntiles = ((N + kBN - 1) / kBN) * ((M + kBM - 1) / kBM);
   for (int kb0 = 0; kb0 < args.KB; kb0 += kKChunkBlocks) {
     args.kb0 = kb0;
@@ -505,7 +507,9 @@ int xs_ozaki_gemm(char transa, char transb, int M, int N, int K, double alpha, c
       args.nops[0] = make_ops(nslices, rows, cols, d0, args.ndiag, true, args.op[0]);
       args.nops[1] = make_ops(nslices, rows, cols, d0, args.ndiag, false, args.op[1]);
       prof = xs_profile_begin(stream);
-      xs_ozaki_gemm_kernel<<<min(ntiles, xs_sm_count()), kGemmThreads, smem, s>>>(args);
+      const auto kernel = (kRegOps >= args.nops[1]) ? &xs_ozaki_gemm_kernel<true> : &xs_ozaki_gemm_kernel<false>;
+      if (0 != (r = xs_func_smem((const void*)kernel, smem))) return r;
+      kernel<<<min(ntiles, xs_sm_count()), kGemmThreads, smem, s>>>(args);
       if (0 != (r = (int)cudaGetLastError())) return r;
       const double kc = (double)(args.kb1 - args.kb0) * kBK;
       xs_profile_end(prof, "ozaki_gemm", 2.0 * M * N * (kc < K ? kc : K), 0.0, stream);
