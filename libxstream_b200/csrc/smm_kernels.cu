@@ -2222,14 +2222,14 @@ __global__ void xs_norms_kernel(const double* __restrict__ mat, int nblks, const
   const int lane = threadIdx.x & 31;
   const int blk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (blk >= nblks) return;
-  const double* const p = mat + offsets[blk];
-  const int ne = nelems[blk];
+  const double* p = mat + offsets[blk] + lane;
   double s = 0.0;
-  /* eight loads in flight: one by one, a block of 22x22 took 15 trips to memory */
-  for (int e = lane; e < ne; e += 8 * 32) {
+  /* eight loads in flight: one by one, a block of 22x22 took 15 trips to memory. Counted down: an index could
+     pass the largest int by the last trip */
+  for (int left = nelems[blk] - lane; left > 0; left -= 8 * 32, p += 8 * 32) {
     double v[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = (e + 32 * u < ne) ? p[e + 32 * u] : 0.0;
+    for (int u = 0; u < 8; ++u) v[u] = (32 * u < left) ? p[32 * u] : 0.0;
 #pragma unroll
     for (int u = 0; u < 8; ++u) s = fma(v[u], v[u], s);
   }

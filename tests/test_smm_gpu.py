@@ -202,6 +202,24 @@ def test_norms(acc):
         b.free()
 
 
+def test_norm_of_the_largest_block(acc):
+    """2^31 - 1 elements (16 GB): the last trips of the loop lie within 256 elements of the largest int."""
+    A, stream = acc
+    n = 2**31 - 1
+    mat = A.DevBuf(8 * n)
+    mat.zero(stream)
+    tail = np.array([3.0, 0.0, 4.0])
+    assert A.lib().c_dbcsr_acc_memcpy_h2d(tail.ctypes.data, mat.ptr + 8 * (n - 3), tail.nbytes, stream.handle) == 0
+    do, dn = A.DevBuf.from_array(np.zeros(1, np.int32), stream), A.DevBuf.from_array(np.array([n], np.int32), stream)
+    dout = A.DevBuf(4)
+    assert A.norms(mat, 1, do, dn, dout, stream) == 0
+    got = dout.download(np.zeros(1, np.float32), stream)
+    stream.sync()
+    assert got[0] == 5.0
+    for b in (mat, do, dn, dout):
+        b.free()
+
+
 def test_unhandled_returns_minus_one_on_device(acc):
     A, stream = acc
     dummy = A.DevBuf(64)
