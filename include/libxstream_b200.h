@@ -73,10 +73,12 @@ double libxstream_b200_fp64_peak(void* stream);
 /** Set the kernel parameters used for FP64 stacks of shape (m, n, k): chunk = entries per warp
     (0: size to each stack), mt/nt = warp sub-tile in 8x8 DMMA tiles (1..4), kp = k-steps per
     register panel (2 or 4), wpb = warps per CTA (1..4). Replaces the OPENCL_LIBSMM_SMM_* tunables
-    (samples/smm/smm_kernel.c:194-278). Returns 0 on success. */
+    (samples/smm/smm_kernel.c:194-278). Stacks of the shape then run as they say, large ones too, which would run on
+    the tile kernel otherwise. Returns 0 on success. */
 int libxstream_b200_set_params(int m, int n, int k, int chunk, int mt, int nt, int kp, int wpb);
 
-/** Read back the parameters used for (m, n, k, stack_size): out6 = {chunk, mt, nt, kp, wpb, sorted}. */
+/** Read back the parameters used for (m, n, k, stack_size): out6 = {chunk, mt, nt, kp, wpb, sorted}. A large stack without
+    a tuned record may run on the tile kernel, which chooses its own tiles (LIBXSTREAM_B200_VERBOSE=3 says so). */
 int libxstream_b200_get_params(int m, int n, int k, int stack_size, int* out6);
 
 /** Forget all tuned parameters (defaults apply afterwards). */

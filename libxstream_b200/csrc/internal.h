@@ -210,9 +210,10 @@ int xs_stack_group(const int* dev_stack, int S, unsigned* k0, unsigned long long
     blk > 0: the C block size (blocks of the stack do not overlap), which spares the gcd statistics.
     heavy > 0: in a single-pass grouping (stacks of at most 65536 entries over at most 2048 block
     positions), the C blocks with at least `heavy` entries come first, then the others, each class in
-    offset order (entries of one block stay in stack order). */
+    offset order (entries of one block stay in stack order). late: a kernel launched behind it with programmatic
+    stream serialization starts when the grouping has ended, not beside it. */
 int xs_stack_group_ex(const int* dev_stack, int S, int format, unsigned blk, unsigned* k0, unsigned long long* v0, unsigned* k1,
-  unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, int* zero, int nzero, int heavy,
+  unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, int* zero, int nzero, int heavy, int late,
   void* sort_scratch, void* stream);
 int xs_stack_group_batch(const xs_sort_batch_t* desc, unsigned* k0, unsigned long long* v0, unsigned* k1,
   unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, void* sort_scratch, void* stream);

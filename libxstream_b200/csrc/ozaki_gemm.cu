@@ -16,14 +16,14 @@
  * of at most 16384 keeps |D_d| < 8 * 16384 * 127^2 < 2^31; longer K runs in chunks of 16384.
  *
  * Device layout: digit panels, the order in which the GEMM reads them. Rows of op(A) in blocks of 128
- * and columns of op(B) in blocks of 64, k in blocks of 32: panel (row block, k block) holds all slices
- * one after the other, each as core matrices of 8 rows x 16 bytes (row group g at 256 g, k half h at
- * 128 h, row r % 8 at 16 (r % 8)); K zero padded; exponents ea[M], eb[N] (int32).
+ * and columns of op(B) in blocks of 64 (one block of 8 or 16 rows' granularity when there are fewer), k in blocks of 32:
+ * panel (row block, k block) holds all slices one after the other, each as core matrices of 8 rows x 16 bytes (row
+ * group g at 256 g, k half h at 128 h, row r % 8 at 16 (r % 8)); K zero padded; exponents ea[M], eb[N] (int32).
  *
  * GEMM kernel: persistent, one CTA per SM, 10 warps, tiles of 128 x 64 of C with ALL anti-diagonals (up to
- * eight at a time: 8 x 64 = 512 tensor-memory columns) accumulated at once. Per k block a stage takes the A
- * and the B panel with one bulk copy each; as the B slices lie one after the other, one tcgen05.mma
- * (M = 128, N = 64 w, K = 32) of A slice sa against the w slices from sb on adds the pairs (sa, sb + i) to
+ * eight at a time: 8 x 64 = 512 tensor-memory columns) accumulated at once. A stage takes the A and the B panels of
+ * as many k blocks as fit 36 KB, one at least, with one bulk copy each; as the B slices lie one after the other, one
+ * tcgen05.mma (M = 128, N = 64 w, K = 32) of A slice sa against the w slices from sb on adds the pairs (sa, sb + i) to
  * diagonals sa + sb + i. So every digit is read once per tile instead of once per pair, and C once:
  * 42 KB per 28 pairs of a 32-wide k block at 7 slices, 47 bytes per cycle and SM (128 x 256 tiles, one pair at a
  * time, took 96, more than the L2 delivers, and added every diagonal into C or tensor memory). Warp 0
@@ -31,8 +31,9 @@
  * finished tile in FP64, smallest weight first, and write C. The MMAs of a tile wait for the epilogue of
  * the one before (tensor memory is full): about 3 % at K = 4096. More than eight diagonals (no trim) run as
  * several launches that add into C.
- * Measured on B200 (whole calls, 7 slices, pairs up to the diagonal, 4096^3): 2549 -> 1776 us, 77 TFLOP/s
- * FP64-equivalent; the tensor pipe is what bounds it (3.85e12 int8 operations in about 1.4 ms, power-capped).
+ * Measured on B200 (whole calls, pairs up to the diagonal, 4096^3; slice-pair tiles -> this): 7 slices 2319 -> 1563 us, 88
+ * TFLOP/s FP64-equivalent, tensor pipe 63 % busy; 4 slices 1034 -> 923, 3 slices 743 -> 674 (with stages of one k block and
+ * MMAs put together by the issuing thread from packed fields 1611, 980, 879: that thread bounds forms of few slices).
  * Every mbarrier wait is bounded: a stalled pipeline ends the kernel with an error status (per-call
  * abort word and the library's device error word) instead of a hang.
  */

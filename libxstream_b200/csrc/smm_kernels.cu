@@ -1614,12 +1614,26 @@ static bool use_tile(int m, int n, int k, int S, const xs_smm_params_t* prm) {
 
 static bool spec_listed(int m, int n, int k, const xs_smm_params_t* prm);
 
-/* The tile kernel's plan of a stack, if it takes it. Teams of 4 x 4 tiles are eight warps per SM, which need four
-   entries each to win over a register kernel compiled for the very shape (64^3 in uniform C blocks: 832 entries
-   40 us against 45, 1173: 48 against 54, 1465: 57 against 59, 2930: 98 against 94; in Zipf ones 1173: 50 against 48). */
+/* The tile kernel's plan of a stack, if it takes it. Beyond use_tile and the shape:
+   - Entries of one short panel (at most 24 DMMA instructions per warp, or two steps of 4 x 4 tiles) with padded columns:
+     up to 65536 entries, up to 32768 for 4 x 4 tiles and blocks of 16 rows or fewer. In longer stacks the copies that the
+     team issues itself cost more than the register kernel's loads, whose start no longer counts: 120000 entries,
+     register kernel and tile kernel, us, 32x50x8 328, 371; 16x42x15 222, 272; 24x32x15 235, 268 (in 16666 of 22x32x16 the
+     tile kernel takes 0.81 of the time).
+   - Teams of 4 x 4 tiles are eight warps per SM; over a register kernel compiled for the very shape (64^3) they win from
+     four entries per team up to twenty, and again where the operands come from HBM. Register kernel and tile kernel, us,
+     uniform C blocks: 832 entries 40, 45; 1173: 48, 54; 1600: 68, 63; 3000: 104, 96; 6000: 171, 169; 12000: 304, 315;
+     30000: 698, 734; 60000: 1383, 1381; 100000: 2409, 2235; 200000: 6201, 4591 (pools of S / 8 blocks, at most 8192; up to
+     60000 entries the register kernel is ahead for pools of any size, at 200000 the tile kernel for pools of more than
+     2000 blocks). */
 static bool plan_tile(int S, int m, int n, int k, const xs_smm_params_t* prm, xs_tile_plan_t* tp) {
   if (!use_tile(m, n, k, S, prm) || 0 != xs_tile_plan(S, m, n, k, tp)) return false;
-  return 12 >= tp->mt * tp->nt || !spec_listed(m, n, k, prm) || S >= 4l * tp->ctas * tp->nteam * xs_sm_count();
+  const int psteps = (min(tp->pk, k) - 1) / 4 + 1, instr = tp->mt * tp->nt * psteps;
+  const bool padded = 4 != tp->Q && (0 == m % 16 || 0 == n % 16), wide = 12 < tp->mt * tp->nt;
+  if (padded && 1 == tp->npan && (24 >= instr || (wide && 2 >= psteps)) && S > (16 >= m || wide ? 32768 : 65536)) return false;
+  if (!wide || !spec_listed(m, n, k, prm)) return true;
+  const long teams = (long)tp->ctas * tp->nteam * xs_sm_count();
+  return S > 65536 || (S >= 4 * teams && S < 20 * teams);
 }
 
 int plan_smm(int S, int m, int n, int k, const xs_smm_params_t* prm, SmmPlan* pl) {
@@ -2380,8 +2394,13 @@ int xs_launch_smm_f64_ex(const int* dev_stack, int S, int format, double alpha, 
   void* const sort_scratch = base + pl.off_sort;
   int* const arrive = (int*)(base + pl.off_arrive);
   void* prof = xs_profile_begin(s);
+  /* Hot C blocks go first, and the stack kernel starts beside the grouping. Not so for longer stacks on the register
+     kernel with several warp tiles per block, which read an operand once per tile: their CTAs lose to an even
+     start behind the grouping (73x72x4 in uniform C blocks, 45000 entries: 361 -> 335 us, 60000: 477 -> 437), and hot
+     blocks apart separate neighbours (60000 in Zipf ones: 512 -> 485 beside the grouping). */
+  const bool plain = S > xs_stack_group_cluster_max() && !pl.tile && 1 < pl.nsub; /* staged and FMA kernels: one tile */
   const int r = xs_stack_group_ex(dev_stack, S, format, (unsigned)(m * n), keys_in, vals_in, keys_tmp, vals_tmp, keys_out,
-    vals_out, seglist, arrive, 3 * pl.ngroups * pl.nsub, pl.tile ? 0 : pl.L * pl.W, sort_scratch, s);
+    vals_out, seglist, arrive, 3 * pl.ngroups * pl.nsub, (pl.tile || plain) ? 0 : pl.L * pl.W, plain ? 1 : 0, sort_scratch, s);
   if (0 != r) return r;
   xs_profile_end(prof, "sort", 0.0, 48.0 * S, s);
   StackTask tk = {};

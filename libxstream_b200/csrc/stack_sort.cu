@@ -561,8 +561,8 @@ template <int E>
 __global__ void __launch_bounds__(kClThreads) xs_stack_group_cluster_kernel(const int* __restrict__ stack, int S, int format,
   unsigned blk, unsigned* __restrict__ k0, unsigned long long* __restrict__ v0, unsigned* __restrict__ k1,
   unsigned long long* __restrict__ v1, unsigned* __restrict__ kout, unsigned long long* __restrict__ vout,
-  int* __restrict__ seglist, int* __restrict__ zero, int nzero, SortCtl* ctl, int heavy, unsigned blk_magic,
-  unsigned long long* __restrict__ stamps) {
+  int* __restrict__ seglist, int* __restrict__ zero, int nzero, SortCtl* ctl, int heavy, int late,
+  unsigned blk_magic, unsigned long long* __restrict__ stamps) {
   namespace cg = cooperative_groups;
   extern __shared__ __align__(16) unsigned char s_dyn[];
   unsigned short (*const s_wc)[kRadix] = reinterpret_cast<unsigned short (*)[kRadix]>(s_dyn);
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(kClThreads) xs_stack_group_cluster_kernel(cons
      kernel after this one start (it reads the caller's stack and pools before its own wait). Hides the launch
      from the call before it: 23x23x23, 30000, back to back 59.3 -> 55.9 us; 3000: 27.2 -> 23.9. */
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" :::);
+  if (0 == late) asm volatile("griddepcontrol.launch_dependents;" :::);
   /* every CTA of the cluster must be running before another one writes into its shared memory: arrive
      now, wait before the first push (the stack loads overlap the barrier) */
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
@@ -871,7 +871,7 @@ int group_launch(const xs_sort_batch_t& desc0, unsigned* k0, unsigned long long*
 template <int E>
 int cluster_group_launch(const int* stack, int S, int format, unsigned blk, unsigned* k0, unsigned long long* v0, unsigned* k1,
   unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, int* zero, int nzero, SortCtl* ctl, int ncta,
-  int heavy, cudaStream_t s, unsigned long long* stamps = nullptr) {
+  int heavy, int late, cudaStream_t s, unsigned long long* stamps = nullptr) {
   static int ok[XS_MAXDEV][kClusterMax + 1]; /* per device and cluster size: 0 unknown, 1 supported, -1 not */
   auto kernel = xs_stack_group_cluster_kernel<E>;
   int* const okp = &ok[xs_device_slot()][ncta];
@@ -904,7 +904,7 @@ int cluster_group_launch(const int* stack, int S, int format, unsigned blk, unsi
   cfg.numAttrs = 2;
   const unsigned blk_magic = (1u < blk) ? (unsigned)((1ull << 32) / blk) : 0u;
   return (int)cudaLaunchKernelEx(&cfg, kernel, stack, S, format, blk, k0, v0, k1, v1, kout, vout, seglist, zero, nzero, ctl, heavy,
-    blk_magic, stamps);
+    late, blk_magic, stamps);
 }
 
 /* Four entries per thread up to 32768 entries, eight up to 65536, where one cluster still beats the
@@ -913,13 +913,13 @@ int cluster_group_launch(const int* stack, int S, int format, unsigned blk, unsi
 constexpr int kClusterLarge = 2;
 int cluster_group_any(const int* stack, int S, int format, unsigned blk, unsigned* k0, unsigned long long* v0, unsigned* k1,
   unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, int* zero, int nzero, SortCtl* ctl, int ncta,
-  int heavy, cudaStream_t s, unsigned long long* stamps = nullptr) {
+  int heavy, int late, cudaStream_t s, unsigned long long* stamps = nullptr) {
   if (S <= kClusterEntries) {
-    return cluster_group_launch<kClE>(stack, S, format, blk, k0, v0, k1, v1, kout, vout, seglist, zero, nzero, ctl, ncta, heavy, s,
-      stamps);
+    return cluster_group_launch<kClE>(stack, S, format, blk, k0, v0, k1, v1, kout, vout, seglist, zero, nzero, ctl, ncta, heavy, late,
+      s, stamps);
   }
   return cluster_group_launch<kClusterLarge * kClE>(stack, S, format, blk, k0, v0, k1, v1, kout, vout, seglist, zero, nzero, ctl,
-    ncta, heavy, s, stamps);
+    ncta, heavy, late, s, stamps);
 }
 
 }  // namespace
@@ -964,17 +964,17 @@ int xs_stack_group_batch(const xs_sort_batch_t* desc, unsigned* k0, unsigned lon
 
 int xs_stack_group(const int* dev_stack, int S, unsigned* k0, unsigned long long* v0, unsigned* k1,
   unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, void* sort_scratch, void* stream) {
-  return xs_stack_group_ex(dev_stack, S, 0, 0u, k0, v0, k1, v1, kout, vout, seglist, nullptr, 0, 0, sort_scratch, stream);
+  return xs_stack_group_ex(dev_stack, S, 0, 0u, k0, v0, k1, v1, kout, vout, seglist, nullptr, 0, 0, 0, sort_scratch, stream);
 }
 
 int xs_stack_group_ex(const int* dev_stack, int S, int format, unsigned blk, unsigned* k0, unsigned long long* v0, unsigned* k1,
-  unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, int* zero, int nzero, int heavy,
+  unsigned long long* v1, unsigned* kout, unsigned long long* vout, int* seglist, int* zero, int nzero, int heavy, int late,
   void* sort_scratch, void* stream) {
   if (0 < S && S <= kClusterLarge * kClusterEntries) { /* one cluster of up to 16 CTAs */
     int ncta = 1;
     while (ncta < kClusterMax && ncta * kClThreads * kClE < S) ncta <<= 1;
     const int r = cluster_group_any(dev_stack, S, format, blk, k0, v0, k1, v1, kout, vout, seglist, zero, nzero,
-      (SortCtl*)sort_scratch, ncta, heavy, (cudaStream_t)stream);
+      (SortCtl*)sort_scratch, ncta, heavy, late, (cudaStream_t)stream);
     if (cudaErrorNotSupported != r) return r; /* else: the cooperative kernel below */
   }
   xs_sort_batch_t d;
@@ -1077,7 +1077,7 @@ int xs_stack_group_profile(const int* dev_stack, int S, unsigned blk, unsigned l
   unsigned long long* st = (unsigned long long*)p; p += 8 * sizeof(unsigned long long) * grid;
   int* seg = (int*)p; p += 256;
   p = (char*)(((uintptr_t)p + 255) & ~(uintptr_t)255);
-  int rc = (0 < ncta) ? cluster_group_any(dev_stack, S, 0, blk, k0, v0, k1, v1, ko, vo, seg, nullptr, 0, (SortCtl*)p, ncta, 0, s, st)
+  int rc = (0 < ncta) ? cluster_group_any(dev_stack, S, 0, blk, k0, v0, k1, v1, ko, vo, seg, nullptr, 0, (SortCtl*)p, ncta, 0, 0, s, st)
                       : cudaErrorNotSupported;
   if (cudaErrorNotSupported == rc) rc = group_launch(d, k0, v0, k1, v1, ko, vo, seg, p, s, st, 1);
   if (0 == rc) rc = (int)cudaMemcpyAsync(host_stamps, st, 8 * sizeof(unsigned long long) * grid, cudaMemcpyDeviceToHost, s);

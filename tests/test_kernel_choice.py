@@ -52,7 +52,9 @@ def test_kinds(acc):
     assert kind(45, 45, 45, 3000) == TILE and kind(45, 45, 45, 1000) == REGISTER  # 7e5 DMMA steps are 1621 entries
     assert kind(23, 23, 23, 3000) == kind(23, 23, 23, 300000) == STAGED
     assert kind(46, 13, 5, 100000) == REGISTER  # 12 DMMA instructions per warp and panel
-    assert kind(64, 64, 64, 1100) == REGISTER and kind(64, 64, 64, 1200) == TILE
+    assert [kind(64, 64, 64, S) for S in (1100, 1200, 5900, 6000, 65536, 65537)] == [REGISTER, TILE, TILE, REGISTER, REGISTER, TILE]
+    for shape, most in (((32, 50, 8), 32768), ((16, 42, 15), 32768), ((24, 32, 15), 65536)):  # one short panel, padded columns
+        assert kind(*shape, most) == TILE and kind(*shape, most + 1) == REGISTER
     assert kind(45, 45, 45, 2000000) == TILE  # in parts
     try:
         record(45, 45, 45, 3, 3, 2, 1)
