@@ -259,9 +259,11 @@ __global__ void __maxnreg__(tile_regs(MT, NT)) xs_smm_tile_kernel(const __grid_c
   prefetch_operands(tk);
   pdl_wait();
   pdl_trigger();
-  /* the grouping failed (or a wait of a team that started earlier): the whole CTA writes nothing. One vote for
-     all threads: the word may change while they read it, and the barriers below count on every warp of a team */
-  if (__syncthreads_or((0 != *(volatile const unsigned*)err) ? 1 : 0)) return;
+  /* the grouping failed (or a wait of a team that started earlier): the team writes nothing. One vote for all its
+     threads: the word may change while they read it, and the barriers below count on every warp of a team */
+  const bool failed = 0 != *(volatile const unsigned*)err;
+  __syncthreads();
+  if (team_any(team + 1, threads, failed)) return;
   const int chunk = blockIdx.x * geo.nteam + team;
   if (chunk >= tk.nchunks) return;
   const int m = tk.m, n = tk.n, k = tk.k, npan = geo.npan;
